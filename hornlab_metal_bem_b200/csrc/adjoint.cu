@@ -671,7 +671,7 @@ extern "C" int hbem_session_set_vertices(hbem_session *h, const float *vertices_
     // Duffy pairs are kept)
     static const double QX[6] = {HBEM_QX0, HBEM_QX1, HBEM_QX2, HBEM_QX3, HBEM_QX4, HBEM_QX5};
     static const double QY[6] = {HBEM_QY0, HBEM_QY1, HBEM_QY2, HBEM_QY3, HBEM_QY4, HBEM_QY5};
-    std::vector<float4> qp((size_t)T * 6), nrm(T), sqp((size_t)T * 6), snrm(T);
+    std::vector<float4> qp((size_t)T * 6), nrm(T), sqp, snrm(T);
     for (int t = 0; t < T; ++t) {
         double P[3][3];
         for (int l = 0; l < 3; ++l) {
@@ -686,11 +686,8 @@ extern "C" int hbem_session_set_vertices(hbem_session *h, const float *vertices_
         }
         nrm[t] = make_float4(s->normals[t], s->normals[T + t], s->normals[2 * T + t], 2.0f * s->areas[t]);
     }
-    for (int i = 0; i < T; ++i) {
-        const int t = s->order[i];
-        for (int q = 0; q < 6; ++q) sqp[(size_t)i * 6 + q] = qp[(size_t)t * 6 + q];
-        snrm[i] = nrm[t];
-    }
+    sorted_points(*s, qp, sqp);
+    for (int i = 0; i < T; ++i) snrm[i] = nrm[s->order[i]];
     HBEM_CUDA(cudaMemcpy(s->d_qp, sqp.data(), sizeof(float4) * sqp.size(), cudaMemcpyHostToDevice));
     HBEM_CUDA(cudaMemcpy(s->d_nrm, snrm.data(), sizeof(float4) * snrm.size(), cudaMemcpyHostToDevice));
     HBEM_CUDA(cudaMemcpy(s->d_fqp, qp.data(), sizeof(float4) * qp.size(), cudaMemcpyHostToDevice));

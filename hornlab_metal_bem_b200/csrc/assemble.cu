@@ -9,21 +9,18 @@
 //     folded into A and b on the device (the reference folds them on the CPU,
 //     main.swift:6498-6561).
 //
-// Kernel design (regular part).  A CTA owns a tile of 32 test triangles
-// (one per lane) x 64 trial triangles (eight per warp, warp-uniform).  The
-// trial tile's quadrature points are staged once in shared memory and read
-// as broadcasts; the test points live in registers.  Each lane evaluates
-// 36 x (1 + images) kernel samples per pair with one rsqrt and one fast
-// sincos of k r (the hardware reduces the argument in turns itself, as
+// The regular part has two kernels: k_regular_sym over unordered triangle
+// pairs (the default, see there) with k_rhs for the right-hand sides, and
+// k_regular over ordered pairs (HBEM_TUNE_ASM_PAIRS = 1): a CTA owns 32 test
+// triangles (one per lane) x 64 trial triangles (eight per warp), evaluates
+// 36 x (1 + images) samples per pair and adds the pair block into a
+// shared-memory accumulator indexed by the tile's distinct dofs, flushed once
+// with red.global.add.  Both take one rsqrt and one fast sincos of k r per
+// sample and wavenumber (the hardware reduces the argument in turns itself, as
 // accurately as the FP32 product k r is; the rounding of that product is the
-// phase error either way), factorises the 3x3
-// basis products (inner sum over trial points first) and adds the pair block
-// into a shared-memory accumulator indexed by the tile's distinct dofs.  The
-// tile is flushed once with red.global.add, which cuts global atomics by the
-// ~25x dof sharing inside a spatially compact (Morton ordered) tile.  Values
-// that come in pairs (the two orders of an unordered pair, the Duffy kernel's
-// two wavenumbers) are accumulated as packed FP32 pairs (FFMA2 / FMUL2 /
-// FADD2: half the instructions, the same rounding per element).
+// phase error either way).  Values that come in pairs (two wavenumbers, or the
+// two orders of an unordered pair) are accumulated as packed FP32 pairs (FFMA2
+// / FMUL2 / FADD2: half the instructions, the same rounding per element).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -61,6 +58,14 @@ struct AsmArgs {
     long long q_stride, lda, a_stride, b_stride;
     long long q_src_stride, b_src_stride;   // between sources' Neumann rows / right-hand sides
     int T, nf, n_src;
+    // unordered pairs: chunks of trial triangles with their distinct dofs, the
+    // row lists of the test tiles, float4 entries of one warp's plane, and the
+    // first wavenumber of the launch
+    const uchar4 *chunk_slot;
+    const int *chunk_off;
+    const int *chunk_cols;
+    const unsigned *gather;
+    int plane, f_base, rhs_block;
     float rw;
     float k[kMaxFreqPerLaunch];
     float ki[kMaxFreqPerLaunch];
@@ -408,105 +413,173 @@ __global__ void __launch_bounds__(kAsmThreads, MINB) k_regular(const __grid_cons
 // double-layer kernel in both orders shares everything but a dot product:
 //   dG/dn_y(x, My) = F(r) (d . M n_sigma),   dG/dn_x(y, Mx) = F(r) (-d . n_tau),
 //   F = e^{ikr} (ik - 1/r) / r^2,  d = My - x,  r = |d| = |Mx - y|
-// (M is an involution and an isometry), and G(r) is the same.  So each
-// unordered pair {tau, sigma} (sorted index tau <= sigma) is evaluated once
-// (the coincident self-point of tau = sigma has r^2 = 0 exactly and drops out
-// through the singular-point guard, as the reference excludes it)
-// and adds A[tau dofs][sigma dofs], A[sigma dofs][tau dofs] and both RHS
-// rows: one rsqrt / sincos per sample instead of two.  Tiles and the shared
-// accumulation are those of k_regular with a second, transposed plane.
+// (M is an involution and an isometry).  So each unordered pair {tau, sigma}
+// (sorted index tau <= sigma) is evaluated once and adds A[tau dofs][sigma
+// dofs] and A[sigma dofs][tau dofs].  d . M n_sigma is the same for every
+// point of the flat triangle M sigma, so it is formed once per test point and
+// image, scaled by both Jacobians.
+//
+// Split.  A warp owns 32 test triangles (one per lane) x a chunk of 8 trial
+// triangles (warp-uniform); 4 such warps share a CTA's test tile.  NF = 2
+// wavenumbers ride in the two halves of packed FP32 pairs (FFMA2 / FMUL2: one
+// instruction for two FP32 operations, each rounded as its scalar twin) and
+// share the geometry and the rsqrt of a sample; NF = 1 packs the two orders.
+//
+// Scatter.  The 3 x 3 blocks of a lane stay in registers while the trial dof
+// of a column slot is shared by consecutive triangles of the chunk (the
+// session orders triangles and their local vertices for that: 1.26 new dofs a
+// triangle); a finished column is staged in shared memory as (forward re, im,
+// transposed re, im) per (lane, test vertex), lane r sums the entries of test
+// row r (at most valence many) and adds the row total to the warp's own plane
+// (rows x chunk dofs), which goes to A with red.global.add once per chunk.
+// No shared-memory atomics: they are compare-and-swap loops in FP32, and with
+// one per block entry their retries took half of the kernel with four images
+// and four fifths of it with one.
+//
+// Bound: issue (a packed instruction takes two slots of the FP32 pipe; 82 % of
+// them busy with one image), with four images the MUFU pipe as well (1 rsqrt
+// + 2 NF per sample: 62 %).  Regular assembly with right-hand sides, 40
+// wavenumbers: quarter horn (1950 triangles, 4 images) 15.8 -> 9.6 ms, half
+// horn (3664, 2 images) 40.0 -> 21.1 ms; full horn (8332, 6 wavenumbers)
+// 26.0 -> 11.7 ms; sphere with every face driven (1280, 8) 2.33 -> 0.72 ms.
+// Two CTAs an SM with 255 registers each were 2-8 % slower than three with 168.
 // ---------------------------------------------------------------------------
-// Without G (NEED_G false) the singular-point guard costs two instructions
-// a sample: there r^2 gets 1e-30 added instead, which leaves r^2 of every
-// distinct point pair unchanged in FP32 and makes the coincident point
-// (d = 0 exactly) contribute exactly 0: its dG/dn terms carry the factor
-// d.n = 0 times a finite 1/r^2 = 1e30.
-// The two orders ride in the two halves of packed FP32 pairs: dr = (dre,
-// tre), di = (dim, tim), one FFMA2 (sm_100: two FP32 FMAs as one
-// instruction, each rounded as its scalar twin) for both orders' D or T.
-template <bool CK, bool NEED_G>
-__device__ __forceinline__ void sample_sym(float dx, float dy, float dz, float nsx, float nsy, float nsz, float ntx,
-                                            float nty, float ntz, float k, float ki, float2 &dr, float2 &di,
-                                            float &gre, float &gim) {
-    const float r2 = NEED_G ? fmaf(dx, dx, fmaf(dy, dy, dz * dz)) : fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, 1.0e-30f)));
-    float u = rsqrtf(r2);
-    if (NEED_G) u = r2 > 1.0e-14f ? u : 0.0f;
-    const float r = r2 * u;
-    const float u2 = u * u;
-    float hs = fmaf(dx, nsx, fmaf(dy, nsy, dz * nsz)) * u2;
-    float ht = -fmaf(dx, ntx, fmaf(dy, nty, dz * ntz)) * u2;
-    float sn, cs;
-    __sincosf(r * k, &sn, &cs);
-    float uu = u, fre = u;
-    if (CK) {
-        const float damp = __expf(-ki * r);
-        hs *= damp;
-        ht *= damp;
-        uu *= damp;
-        fre += ki;
-    }
-    const float e_re = -fmaf(cs, fre, sn * k), e_im = fmaf(cs, k, -sn * fre);
-    const float2 h2 = make_float2(hs, ht);
-    dr = __ffma2_rn(h2, make_float2(e_re, e_re), dr);
-    di = __ffma2_rn(h2, make_float2(e_im, e_im), di);
-    if (NEED_G) {
-        gre = fmaf(uu, cs, gre);
-        gim = fmaf(uu, sn, gim);
-    }
+constexpr int kPairWarps = 4;
+
+__device__ __forceinline__ float rsqrt_ftz(float x) {
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
 }
 
-// One unordered pair, one wavenumber.  Outputs (times 1/(4 pi) and the
-// Jacobians later): fwd[i*3+j] test dof i x trial dof j, trn[j*3+i] trial dof j
-// x test dof i; SLP rows sfw[i] (test) and str[j] (trial, summed with the
-// test-point weights only).
-template <int SYM, bool CK, bool NEED_G>
-__device__ __forceinline__ void pair_block_sym(const float4 *__restrict__ tq, const float4 *__restrict__ sp, float nx,
-                                               float ny, float nz, float tnx, float tny, float tnz, float k, float ki,
-                                               float (&fwr)[9], float (&fwi)[9], float (&tnr)[9],
-                                               float (&tni)[9], float (&sfr)[3], float (&sfi)[3], float (&str_)[3],
-                                               float (&sti)[3]) {
-    float2 Fr[9], Fi[9];   // (fwd[i*3+j], trn[j*3+i])
-#pragma unroll
-    for (int i = 0; i < 9; ++i) Fr[i] = Fi[i] = make_float2(0.f, 0.f);
-#pragma unroll
-    for (int i = 0; i < 3; ++i) sfr[i] = sfi[i] = str_[i] = sti[i] = 0.0f;
-#pragma unroll 1
+__device__ __forceinline__ float2 dup2(float x) { return make_float2(x, x); }
+
+// Signs of image m (0: the triangle itself) of symmetry SYM
+template <int SYM>
+__host__ __device__ constexpr int n_images() { return SYM == 0 ? 1 : (SYM == 3 ? 4 : 2); }
+template <int SYM>
+__device__ __forceinline__ constexpr int image_mask(int m) {
+    return m == 0 ? 0 : (SYM == 3 ? m : SYM);
+}
+__device__ __forceinline__ constexpr float sgn(int mask, int axis) { return (mask >> axis) & 1 ? -1.f : 1.f; }
+
+// Block accumulators of a lane: [i * 3 + slot] test vertex i, trial slot.
+// NF = 2: forward and transposed entries, (first, second wavenumber);
+// NF = 1: (forward, transposed).
+template <int NF>
+struct PairAcc {
+    float2 r[NF][9], i[NF][9];
+};
+
+// One unordered pair accumulated into acc.  hn is the scaled trial normal
+// (times -1), tn the scaled test normal; both zero for a lane whose pair does
+// not count.  drop0: the pair of a triangle with itself (its own plane: no
+// double layer, and no transposed block).
+template <int SYM, bool CK, int NF, bool ROBIN>
+__device__ __forceinline__ void pair_accumulate(const float4 *__restrict__ tq, const float4 *__restrict__ sp, float hx,
+                                                float hy, float hz, float tnx, float tny, float tnz, bool self,
+                                                float2 k2, float2 nk2, float2 ki2, PairAcc<NF> &acc, float (&sfr)[3],
+                                                float (&sfi)[3], float (&str_)[3], float (&sti)[3]) {
+    constexpr int M = n_images<SYM>();
+    // The test-point loop stays rolled (test point from shared memory, weights
+    // from constant memory) so the kernel body fits the instruction cache; the
+    // trial-point loop is unrolled with the image samples.  Two test points at
+    // a time pay with two images only (half horn of 3664 triangles x 40
+    // wavenumbers 21.9 -> 21.1 ms; one image 11.7 -> 12.1 ms).
+#pragma unroll(M == 2 ? 2 : 1)
     for (int a = 0; a < 6; ++a) {
         const float4 x = tq[a * kTestTile];
-        float2 er[3], ei[3];
+        float hp[M];   // -scale (M y - x) . M n_sigma, the same for every y of the triangle
+        {
+            const float4 y = sp[0];
+#pragma unroll
+            for (int m = 0; m < M; ++m) {
+                const int mk = image_mask<SYM>(m);
+                hp[m] = fmaf(sgn(mk, 0) * y.x - x.x, sgn(mk, 0) * hx,
+                             fmaf(sgn(mk, 1) * y.y - x.y, sgn(mk, 1) * hy, (sgn(mk, 2) * y.z - x.z) * (sgn(mk, 2) * hz)));
+            }
+            if (self) hp[0] = 0.f;
+        }
+        float2 er[NF][3], ei[NF][3];   // NF = 2: [0] forward, [1] transposed
         float hre = 0.f, him = 0.f, g2r[3], g2i[3];
 #pragma unroll
-        for (int j = 0; j < 3; ++j) { er[j] = ei[j] = make_float2(0.f, 0.f); g2r[j] = g2i[j] = 0.f; }
+        for (int j = 0; j < 3; ++j) {
+#pragma unroll
+            for (int o = 0; o < NF; ++o) er[o][j] = ei[o][j] = make_float2(0.f, 0.f);
+            g2r[j] = g2i[j] = 0.f;
+        }
 #pragma unroll
         for (int b = 0; b < 6; ++b) {
             const float4 y = sp[b];
-            float2 dr = make_float2(0.f, 0.f), di = make_float2(0.f, 0.f);
+            float2 dr[NF], di[NF];
             float gre = 0.f, gim = 0.f;
-            sample_sym<CK, NEED_G>(y.x - x.x, y.y - x.y, y.z - x.z, nx, ny, nz, tnx, tny, tnz, k, ki, dr, di, gre, gim);
-            if (SYM == 1 || SYM == 3)
-                sample_sym<CK, NEED_G>(-y.x - x.x, y.y - x.y, y.z - x.z, -nx, ny, nz, tnx, tny, tnz, k, ki,
-                                       dr, di, gre, gim);
-            if (SYM == 2 || SYM == 3)
-                sample_sym<CK, NEED_G>(y.x - x.x, -y.y - x.y, y.z - x.z, nx, -ny, nz, tnx, tny, tnz, k, ki,
-                                       dr, di, gre, gim);
-            if (SYM == 3)
-                sample_sym<CK, NEED_G>(-y.x - x.x, -y.y - x.y, y.z - x.z, -nx, -ny, nz, tnx, tny, tnz, k, ki,
-                                       dr, di, gre,
-                                        gim);
-            if (SYM == 4)
-                sample_sym<CK, NEED_G>(y.x - x.x, y.y - x.y, -y.z - x.z, nx, ny, -nz, tnx, tny, tnz, k, ki,
-                                       dr, di, gre, gim);
+#pragma unroll
+            for (int o = 0; o < NF; ++o) dr[o] = di[o] = make_float2(0.f, 0.f);
+#pragma unroll
+            for (int m = 0; m < M; ++m) {
+                const int mk = image_mask<SYM>(m);
+                const float dx = sgn(mk, 0) * y.x - x.x, dy = sgn(mk, 1) * y.y - x.y, dz = sgn(mk, 2) * y.z - x.z;
+                // 1e-30 leaves r^2 of distinct points unchanged in FP32 and
+                // keeps the coincident point finite (its factors are 0)
+                const float r2 = fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, 1.0e-30f)));
+                const float u = rsqrt_ftz(r2);
+                const float r = r2 * u, u2 = u * u;
+                const float hh = hp[m] * u2;
+                const float tt = fmaf(dx, tnx, fmaf(dy, tny, dz * tnz)) * u2;
+                // P + i Q = -e^{ikr} (ik - 1/r), with k = k + i ki
+                if constexpr (NF == 2) {
+                    const float2 ph = __fmul2_rn(dup2(r), k2);
+                    float2 sn, cs;
+                    __sincosf(ph.x, &sn.x, &cs.x);
+                    __sincosf(ph.y, &sn.y, &cs.y);
+                    float2 fre = dup2(u);
+                    if (CK) {
+                        const float2 damp = make_float2(__expf(-ki2.x * r), __expf(-ki2.y * r));
+                        sn = __fmul2_rn(sn, damp);
+                        cs = __fmul2_rn(cs, damp);
+                        fre = __fadd2_rn(fre, ki2);
+                    }
+                    const float2 P = __ffma2_rn(cs, fre, __fmul2_rn(sn, k2));
+                    const float2 Q = __ffma2_rn(sn, fre, __fmul2_rn(cs, nk2));
+                    const float2 h2 = dup2(hh), t2 = dup2(tt);
+                    dr[0] = __ffma2_rn(P, h2, dr[0]);
+                    di[0] = __ffma2_rn(Q, h2, di[0]);
+                    dr[NF - 1] = __ffma2_rn(P, t2, dr[NF - 1]);
+                    di[NF - 1] = __ffma2_rn(Q, t2, di[NF - 1]);
+                } else {
+                    float sn, cs, fre = u;
+                    __sincosf(r * k2.x, &sn, &cs);
+                    if (CK) {
+                        const float damp = __expf(-ki2.x * r);
+                        sn *= damp;
+                        cs *= damp;
+                        fre += ki2.x;
+                    }
+                    const float P = fmaf(cs, fre, sn * k2.x), Q = fmaf(sn, fre, cs * nk2.x);
+                    const float2 h2 = make_float2(hh, tt);
+                    dr[0] = __ffma2_rn(h2, dup2(P), dr[0]);
+                    di[0] = __ffma2_rn(h2, dup2(Q), di[0]);
+                    if (ROBIN) {
+                        const float ug = r2 > 1.0e-14f ? u : 0.0f;
+                        gre = fmaf(ug, cs, gre);
+                        gim = fmaf(ug, sn, gim);
+                    }
+                }
+            }
 #pragma unroll
             for (int j = 0; j < 3; ++j) {
                 const float wb = qw(b) * bas(b, j);
-                er[j] = __ffma2_rn(dr, make_float2(wb, wb), er[j]);
-                ei[j] = __ffma2_rn(di, make_float2(wb, wb), ei[j]);
-                if (NEED_G) {
+#pragma unroll
+                for (int o = 0; o < NF; ++o) {
+                    er[o][j] = __ffma2_rn(dr[o], dup2(wb), er[o][j]);
+                    ei[o][j] = __ffma2_rn(di[o], dup2(wb), ei[o][j]);
+                }
+                if (ROBIN) {
                     g2r[j] = fmaf(gre, wb, g2r[j]);
                     g2i[j] = fmaf(gim, wb, g2i[j]);
                 }
             }
-            if (NEED_G) {
+            if (ROBIN) {
                 hre = fmaf(gre, qw(b), hre);
                 him = fmaf(gim, qw(b), him);
             }
@@ -515,16 +588,18 @@ __device__ __forceinline__ void pair_block_sym(const float4 *__restrict__ tq, co
         for (int i = 0; i < 3; ++i) {
             const float2 wa = c_wa2[a][i];
 #pragma unroll
-            for (int j = 0; j < 3; ++j) {
-                Fr[i * 3 + j] = __ffma2_rn(wa, er[j], Fr[i * 3 + j]);
-                Fi[i * 3 + j] = __ffma2_rn(wa, ei[j], Fi[i * 3 + j]);
-            }
-            if (NEED_G) {
+            for (int j = 0; j < 3; ++j)
+#pragma unroll
+                for (int o = 0; o < NF; ++o) {
+                    acc.r[o][i * 3 + j] = __ffma2_rn(wa, er[o][j], acc.r[o][i * 3 + j]);
+                    acc.i[o][i * 3 + j] = __ffma2_rn(wa, ei[o][j], acc.i[o][i * 3 + j]);
+                }
+            if (ROBIN) {
                 sfr[i] = fmaf(wa.x, hre, sfr[i]);
                 sfi[i] = fmaf(wa.x, him, sfi[i]);
             }
         }
-        if (NEED_G) {
+        if (ROBIN) {
             const float wq = c_w[a];
 #pragma unroll
             for (int j = 0; j < 3; ++j) {
@@ -533,237 +608,460 @@ __device__ __forceinline__ void pair_block_sym(const float4 *__restrict__ tq, co
             }
         }
     }
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-            fwr[i * 3 + j] = Fr[i * 3 + j].x;
-            tnr[j * 3 + i] = Fr[i * 3 + j].y;
-            fwi[i * 3 + j] = Fi[i * 3 + j].x;
-            tni[j * 3 + i] = Fi[i * 3 + j].y;
-        }
 }
 
-// blockIdx.z = frequency.  CTAs whose test triangles all follow their trial
-// triangles in the sorted order have no unordered pair of their own and exit.
-template <int SYM, bool CK, int MINB>
-__global__ void __launch_bounds__(kAsmThreads, MINB) k_regular_sym(const __grid_constant__ AsmArgs p) {
-    extern __shared__ float2 s_acc[];
-    __shared__ float4 s_qp[kTrialTile * 6];
+// blockIdx.z = group of NF wavenumbers starting at f_base.  CTAs and warps
+// whose test triangles all follow their trial triangles have no pair of their
+// own and do nothing.  Dynamic shared memory: kPairWarps planes of
+// NF x max chunk dofs x (max rows | 1) float4.
+template <int SYM, bool CK, int NF, bool ROBIN>
+__global__ void __launch_bounds__(kPairWarps * 32, NF == 2 ? 3 : 4) k_regular_sym(const __grid_constant__ AsmArgs p) {
+    extern __shared__ float4 s_plane[];
+    __shared__ float4 s_qp[kPairWarps][kChunk * 6];
     __shared__ float4 s_tq[kTestTile * 6];
-    __shared__ float4 s_nrm[kTrialTile];
-    __shared__ uchar4 s_cs[kTrialTile];
-    __shared__ float2 s_q[kMaxSources][kTrialTile];    // Neumann data of the trial triangles per source
-    __shared__ float2 s_tqq[kMaxSources][kTestTile];   // ... and of the test triangles
-    __shared__ float2 s_beta[kTrialTile];
-    __shared__ int s_flag[kTrialTile];
+    __shared__ float4 s_nrm[kPairWarps][kChunk];
+    __shared__ uchar4 s_cs[kPairWarps][kChunk];
+    __shared__ float2 s_beta[ROBIN ? kPairWarps : 1][kChunk];
+    __shared__ float4 s_stage[kPairWarps][NF][3 * kTestTile + 1];
+    __shared__ __align__(16) unsigned char s_gl[kGatherBytes];   // row -> (lane, vertex) lists of the test tile
+    __shared__ int s_rows[3 * kTestTile];
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int f = blockIdx.z;
-    const int test_tile = blockIdx.y, trial_tile = blockIdx.x;
+    const int f0 = p.f_base + blockIdx.z * NF;
+    const int test0 = blockIdx.y * kTestTile;
     const int T = p.T;
-    const int tbase = trial_tile * kTrialTile;
-    const int ntrial = min(kTrialTile, T - tbase);
-    const int test0 = test_tile * kTestTile;
+    if (test0 > blockIdx.x * (kPairWarps * kChunk) + kPairWarps * kChunk - 1) return;
     const int ntest = min(kTestTile, T - test0);
-    if (test0 > tbase + ntrial - 1) return;   // every test triangle follows every trial triangle
-    const int r0 = p.row_off[test_tile], nrows = p.row_off[test_tile + 1] - r0;
-    const int c0 = p.col_off[trial_tile], ncols = p.col_off[trial_tile + 1] - c0;
-    const int ldc = ncols | 1, ldr = nrows | 1;
-    const int nsrc = p.n_src;
-    float2 *acc = s_acc;                       // nrows x ldc   (test rows, trial columns)
-    float2 *rhs = acc + nrows * ldc;           // nsrc x nrows
-    float2 *acc2 = rhs + nsrc * nrows;         // ncols x ldr   (trial rows, test columns)
-    float2 *rhs2 = acc2 + ncols * ldr;         // nsrc x ncols
-    const int plane = nrows * ldc + nsrc * nrows + ncols * ldr + nsrc * ncols;
+    const int r0 = p.row_off[blockIdx.y], nrows = p.row_off[blockIdx.y + 1] - r0;
+    const int chunk = blockIdx.x * kPairWarps + warp;
+    const int tbase = chunk * kChunk;
+    const int ntrial = min(kChunk, T - tbase);   // <= 0: no triangles
+    const bool work = ntrial > 0 && test0 <= tbase + ntrial - 1;
 
-    for (int i = tid; i < plane; i += kAsmThreads) s_acc[i] = make_float2(0.f, 0.f);
-    for (int i = tid; i < ntrial * 6; i += kAsmThreads) s_qp[i] = p.qp[(size_t)tbase * 6 + i];
-    for (int i = tid; i < ntest * 6; i += kAsmThreads) {
+    for (int i = tid; i < kTestTile * 6; i += kPairWarps * 32) {
         const int t = i / 6, a = i - 6 * t;
-        s_tq[a * kTestTile + t] = p.qp[(size_t)(test0 + t) * 6 + a];
+        s_tq[a * kTestTile + t] = p.qp[(size_t)min(test0 + t, T - 1) * 6 + a];
     }
-    for (int i = tid; i < ntrial; i += kAsmThreads) {
-        s_nrm[i] = p.nrm[tbase + i];
-        s_cs[i] = p.trial_slot[tbase + i];
-        const int orig = p.tri[tbase + i].w;
-        int flag = 0;
-        for (int sv = 0; sv < nsrc; ++sv) {
-            float2 qv = make_float2(0.f, 0.f);
-            if (p.q_re) {
-                const size_t o = (size_t)sv * p.q_src_stride + (size_t)f * p.q_stride + orig;
-                qv = make_float2(p.q_re[o], p.q_im[o]);
+    for (int i = tid; i < kGatherBytes / 4; i += kPairWarps * 32)
+        reinterpret_cast<unsigned *>(s_gl)[i] = p.gather[(size_t)blockIdx.y * (kGatherBytes / 4) + i];
+    for (int i = tid; i < nrows; i += kPairWarps * 32) s_rows[i] = p.rows[r0 + i];
+    const int ldr = nrows | 1;
+    int c0 = 0, ncols = 0;
+    float4 *plane = s_plane + (size_t)warp * NF * p.plane;
+    if (work) {
+        c0 = p.chunk_off[chunk];
+        ncols = p.chunk_off[chunk + 1] - c0;
+        for (int i = lane; i < NF * p.plane; i += 32) plane[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int i = lane; i < ntrial * 6; i += 32) s_qp[warp][i] = p.qp[(size_t)tbase * 6 + i];
+        if (lane < ntrial) {
+            s_nrm[warp][lane] = p.nrm[tbase + lane];
+            s_cs[warp][lane] = p.chunk_slot[tbase + lane];
+            if (ROBIN) {
+                const int orig = p.tri[tbase + lane].w;
+                s_beta[warp][lane] = make_float2(p.beta_re[orig], p.beta_im[orig]);
             }
-            s_q[sv][i] = qv;
-            flag |= (qv.x != 0.f || qv.y != 0.f) ? 1 : 0;
         }
-        const float2 be = p.beta_re ? make_float2(p.beta_re[orig], p.beta_im[orig]) : make_float2(0.f, 0.f);
-        s_beta[i] = be;
-        s_flag[i] = flag | ((be.x != 0.f || be.y != 0.f) ? 1 : 0);
-    }
-    for (int i = tid; i < nsrc * ntest; i += kAsmThreads) {
-        const int sv = i / ntest, t = i - sv * ntest;
-        float2 qv = make_float2(0.f, 0.f);
-        if (p.q_re) {
-            const size_t o = (size_t)sv * p.q_src_stride + (size_t)f * p.q_stride + p.tri[test0 + t].w;
-            qv = make_float2(p.q_re[o], p.q_im[o]);
-        }
-        s_tqq[sv][t] = qv;
+        if (lane < NF) s_stage[warp][lane][3 * kTestTile] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
     __syncthreads();
+    if (!work) return;
 
-    const float k = p.k[f], ki = p.ki[f];
-    const int test = test0 + lane;
-    if (lane < ntest) {
-        const float4 tn = p.nrm[test];
-        const float tjac = tn.w;
-        const uchar4 rs = p.test_slot[test];
-        const int rslot[3] = {rs.x, rs.y, rs.z};
+    const int f1 = min(f0 + NF - 1, p.nf - 1);
+    const float2 k2 = make_float2(p.k[f0], p.k[f1]), nk2 = make_float2(-k2.x, -k2.y);
+    const float2 ki2 = make_float2(p.ki[f0], p.ki[f1]);
+    const int test = min(test0 + lane, T - 1);
+    const bool live = lane < ntest;
+    const float4 tn = p.nrm[test];
+    const float tscale = HBEM_INV4PI * p.rw * tn.w;
+    float2 tbe = make_float2(0.f, 0.f);
+    if (ROBIN) {
         const int torig = p.tri[test].w;
-        const float2 tbe = p.beta_re ? make_float2(p.beta_re[torig], p.beta_im[torig]) : make_float2(0.f, 0.f);
-        bool tflag = tbe.x != 0.f || tbe.y != 0.f;
-        for (int sv = 0; sv < nsrc; ++sv) tflag |= s_tqq[sv][lane].x != 0.f || s_tqq[sv][lane].y != 0.f;
-        const float4 *tq = &s_tq[lane];
-        // i k beta / 3 terms: Robin rows of the trial (forward) and test (transposed) triangles
-        auto robin = [&](float br, float bi, float &rr, float &ri) {
-            rr = 0.f;
-            ri = 0.f;
-            if (br != 0.f || bi != 0.f) {
-                const float ikb_re = -ki * br - k * bi;
-                const float ikb_im = -ki * bi + k * br;
-                rr = -ikb_re * (1.0f / 3.0f);
-                ri = -ikb_im * (1.0f / 3.0f);
-            }
-        };
-        float rob2_re, rob2_im;
-        robin(tbe.x, tbe.y, rob2_re, rob2_im);
-        for (int jj = warp; jj < ntrial; jj += kAsmThreads / 32) {
-            const int sigma = tbase + jj;
-            if (sigma < test) continue;
-            const float4 nj = s_nrm[jj];
-            const bool self = sigma == test;
-            float fwr[9], fwi[9], tnr[9], tni[9], sfr[3], sfi[3], str_[3], sti[3];
-            if (s_flag[jj] || tflag)
-                pair_block_sym<SYM, CK, true>(tq, &s_qp[jj * 6], nj.x, nj.y, nj.z, tn.x, tn.y, tn.z, k, ki,
-                                              fwr, fwi, tnr, tni, sfr, sfi, str_, sti);
-            else
-                pair_block_sym<SYM, CK, false>(tq, &s_qp[jj * 6], nj.x, nj.y, nj.z, tn.x, tn.y, tn.z, k, ki,
-                                               fwr, fwi, tnr, tni, sfr, sfi, str_, sti);
-            const float scale = HBEM_INV4PI * tjac * nj.w;
-            const uchar4 cs = s_cs[jj];
-            const int cslot[3] = {cs.x, cs.y, cs.z};
-            const float2 be = s_beta[jj];
-            float rob_re, rob_im;
-            robin(be.x, be.y, rob_re, rob_im);
+        tbe = make_float2(p.beta_re[torig], p.beta_im[torig]);
+    }
+    // -(1/3) i k beta: Robin rows of the trial (forward) and test (transposed) triangles
+    auto robin = [&](float2 be) {
+        const float ikb_re = -ki2.x * be.x - k2.x * be.y, ikb_im = -ki2.x * be.y + k2.x * be.x;
+        return make_float2(-ikb_re * (1.0f / 3.0f), -ikb_im * (1.0f / 3.0f));
+    };
+    // this lane's row of the tile: its first eight contributions packed (the
+    // zero entry 3 * kTestTile pads), the rest from the list in shared memory
+    unsigned g_lo = 0, g_hi = 0;
+    int g_more = 0;   // contributions beyond eight
+    {
+        const int o = lane < nrows ? s_gl[lane] : 0, n = lane < nrows ? s_gl[lane + 1] - o : 0;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            g_lo |= (unsigned)(c < n ? s_gl[kGatherList + o + c] : 3 * kTestTile) << (8 * c);
+            g_hi |= (unsigned)(c + 4 < n ? s_gl[kGatherList + o + c + 4] : 3 * kTestTile) << (8 * c);
+        }
+        g_more = max(0, n - 8);
+    }
+    const int g_max = min(8, __reduce_max_sync(0xffffffffu, lane < nrows ? (int)s_gl[lane + 1] - (int)s_gl[lane] : 0));
+
+    PairAcc<NF> acc;
+#pragma unroll
+    for (int o = 0; o < NF; ++o)
+#pragma unroll
+        for (int e = 0; e < 9; ++e) acc.r[o][e] = acc.i[o][e] = make_float2(0.f, 0.f);
+
+    float4 (*stage)[3 * kTestTile + 1] = s_stage[warp];
+#pragma unroll 1
+    for (int jj = 0; jj < ntrial; ++jj) {
+        const int sigma = tbase + jj;
+        const float4 nj = s_nrm[warp][jj];
+        const uchar4 cs = s_cs[warp][jj];
+        const bool self = sigma == test0 + lane;
+        const float scale = live && sigma >= test0 + lane ? tscale * nj.w : 0.f;
+        const float ts = self ? 0.f : scale;
+        float sfr[3] = {0.f, 0.f, 0.f}, sfi[3] = {0.f, 0.f, 0.f}, str_[3] = {0.f, 0.f, 0.f}, sti[3] = {0.f, 0.f, 0.f};
+        pair_accumulate<SYM, CK, NF, ROBIN>(&s_tq[lane], &s_qp[warp][jj * 6], -scale * nj.x, -scale * nj.y,
+                                            -scale * nj.z, ts * tn.x, ts * tn.y, ts * tn.z, self, k2, nk2, ki2, acc,
+                                            sfr, sfi, str_, sti);
+        if (self) {   // -1/2 mass matrix of the triangle
+            const float m0 = 0.25f * tn.w * p.rw;
+#pragma unroll
+            for (int i = 0; i < 3; ++i)
+#pragma unroll
+                for (int j = 0; j < 3; ++j) {
+                    const float m = m0 * (i == j ? (1.0f / 6.0f) : (1.0f / 12.0f));
+                    acc.r[0][i * 3 + j].x -= m;
+                    if (NF == 2) acc.r[0][i * 3 + j].y -= m;
+                }
+        }
+        if (ROBIN) {
+            const float2 rf = robin(s_beta[warp][jj]), rt = robin(tbe);
 #pragma unroll
             for (int i = 0; i < 3; ++i) {
                 const float s_re = sfr[i] * scale, s_im = sfi[i] * scale;
-                const float radd_re = rob_re * s_re - rob_im * s_im;
-                const float radd_im = rob_re * s_im + rob_im * s_re;
+                const float a_re = rf.x * s_re - rf.y * s_im, a_im = rf.x * s_im + rf.y * s_re;
 #pragma unroll
                 for (int j = 0; j < 3; ++j) {
-                    float vre = fwr[i * 3 + j] * scale + radd_re;
-                    float vim = fwi[i * 3 + j] * scale + radd_im;
-                    if (self) vre -= 0.25f * tjac * (i == j ? (1.0f / 6.0f) : (1.0f / 12.0f));
-                    float2 *dst = &acc[rslot[i] * ldc + cslot[j]];
-                    atomicAdd(&dst->x, vre * p.rw);
-                    atomicAdd(&dst->y, vim * p.rw);
-                }
-#pragma unroll 1
-                for (int sv = 0; sv < nsrc; ++sv) {
-                    const float2 qv = s_q[sv][jj];
-                    if (qv.x != 0.f || qv.y != 0.f) {
-                        atomicAdd(&rhs[sv * nrows + rslot[i]].x, (s_re * qv.x - s_im * qv.y) * p.rw);
-                        atomicAdd(&rhs[sv * nrows + rslot[i]].y, (s_re * qv.y + s_im * qv.x) * p.rw);
-                    }
-                }
-            }
-            if (self) continue;
-#pragma unroll
-            for (int j = 0; j < 3; ++j) {
-                const float s_re = str_[j] * scale, s_im = sti[j] * scale;
-                const float radd_re = rob2_re * s_re - rob2_im * s_im;
-                const float radd_im = rob2_re * s_im + rob2_im * s_re;
-#pragma unroll
-                for (int i = 0; i < 3; ++i) {
-                    const float vre = tnr[j * 3 + i] * scale + radd_re;
-                    const float vim = tni[j * 3 + i] * scale + radd_im;
-                    float2 *dst = &acc2[cslot[j] * ldr + rslot[i]];
-                    atomicAdd(&dst->x, vre * p.rw);
-                    atomicAdd(&dst->y, vim * p.rw);
-                }
-#pragma unroll 1
-                for (int sv = 0; sv < nsrc; ++sv) {
-                    const float2 qv = s_tqq[sv][lane];
-                    if (qv.x != 0.f || qv.y != 0.f) {
-                        atomicAdd(&rhs2[sv * ncols + cslot[j]].x, (s_re * qv.x - s_im * qv.y) * p.rw);
-                        atomicAdd(&rhs2[sv * ncols + cslot[j]].y, (s_re * qv.y + s_im * qv.x) * p.rw);
-                    }
+                    const float t_re = str_[j] * ts, t_im = sti[j] * ts;
+                    acc.r[0][i * 3 + j].x += a_re;
+                    acc.i[0][i * 3 + j].x += a_im;
+                    acc.r[0][i * 3 + j].y += rt.x * t_re - rt.y * t_im;
+                    acc.i[0][i * 3 + j].y += rt.x * t_im + rt.y * t_re;
                 }
             }
         }
+        // finished column slots: stage, sum per test row, add to the plane
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            if (!(cs.w >> j & 1)) continue;   // the next triangle has the same dof in this slot
+            const int col = j == 0 ? cs.x : (j == 1 ? cs.y : cs.z);
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                float2 &r = acc.r[0][i * 3 + j], &im = acc.i[0][i * 3 + j];
+                if constexpr (NF == 2) {
+                    float2 &tr = acc.r[NF - 1][i * 3 + j], &ti = acc.i[NF - 1][i * 3 + j];
+                    stage[0][i * kTestTile + lane] = make_float4(r.x, im.x, tr.x, ti.x);
+                    stage[NF - 1][i * kTestTile + lane] = make_float4(r.y, im.y, tr.y, ti.y);
+                    tr = ti = make_float2(0.f, 0.f);
+                } else {
+                    stage[0][i * kTestTile + lane] = make_float4(r.x, im.x, r.y, im.y);
+                }
+                r = im = make_float2(0.f, 0.f);
+            }
+            __syncwarp();
+            float2 va[NF], vb[NF];
+#pragma unroll
+            for (int o = 0; o < NF; ++o) va[o] = vb[o] = make_float2(0.f, 0.f);
+            auto take = [&](int e) {
+#pragma unroll
+                for (int o = 0; o < NF; ++o) {
+                    const float4 v = stage[o][e];
+                    va[o] = __fadd2_rn(va[o], make_float2(v.x, v.y));
+                    vb[o] = __fadd2_rn(vb[o], make_float2(v.z, v.w));
+                }
+            };
+            auto put = [&](int r) {
+#pragma unroll
+                for (int o = 0; o < NF; ++o) {
+                    float4 &d = plane[o * p.plane + col * ldr + r];
+                    float4 v = d;
+                    v.x += va[o].x;
+                    v.y += va[o].y;
+                    v.z += vb[o].x;
+                    v.w += vb[o].y;
+                    d = v;
+                }
+            };
+            unsigned lo = g_lo, hi = g_hi;
+#pragma unroll 2
+            for (int c = 0; c < g_max; ++c) {
+                take(lo & 255u);
+                lo = __funnelshift_r(lo, hi, 8);
+                hi >>= 8;
+            }
+            if (lane < nrows) {
+                const int o = s_gl[lane];
+                for (int c = 0; c < g_more; ++c) take(s_gl[kGatherList + o + 8 + c]);
+                put(lane);
+            }
+            for (int r = lane + 32; r < nrows; r += 32) {   // tiles of more than 32 distinct dofs
+#pragma unroll
+                for (int o = 0; o < NF; ++o) va[o] = vb[o] = make_float2(0.f, 0.f);
+                for (int c = s_gl[r]; c < s_gl[r + 1]; ++c) take(s_gl[kGatherList + c]);
+                put(r);
+            }
+            __syncwarp();
+        }
     }
-    __syncthreads();
 
-    float *are_g = p.a_re + (size_t)f * p.a_stride;
-    float *aim_g = p.a_im + (size_t)f * p.a_stride;
-    for (int e = tid; e < nrows * ncols; e += kAsmThreads) {
-        const int r = e / ncols, c = e - r * ncols;
-        const float2 v = acc[r * ldc + c];
-        if (v.x != 0.f || v.y != 0.f) {
-            const size_t off = (size_t)p.rows[r0 + r] * p.lda + p.cols[c0 + c];
-            atomicAdd(are_g + off, v.x);
-            atomicAdd(aim_g + off, v.y);
-        }
-    }
-    for (int e = tid; e < ncols * nrows; e += kAsmThreads) {
-        const int c = e / nrows, r = e - c * nrows;
-        const float2 v = acc2[c * ldr + r];
-        if (v.x != 0.f || v.y != 0.f) {
-            const size_t off = (size_t)p.cols[c0 + c] * p.lda + p.rows[r0 + r];
-            atomicAdd(are_g + off, v.x);
-            atomicAdd(aim_g + off, v.y);
-        }
-    }
-    if (p.q_re) {
-        for (int e = tid; e < nsrc * nrows; e += kAsmThreads) {
-            const int sv = e / nrows, r = e - sv * nrows;
-            const float2 v = rhs[e];
+    // the warp's plane into A: forward entries along the chunk's dofs,
+    // transposed ones along the test rows
+    const int *cols = p.chunk_cols + c0;
+    const int total = nrows * ncols;
+    // e / ncols and e / nrows by a 20-bit reciprocal: exact while e times the
+    // divisor stays below 2^20 (at most 24 x 96 entries)
+    const unsigned inv_c = (1u << 20) / ncols + 1, inv_r = (1u << 20) / nrows + 1;
+#pragma unroll
+    for (int o = 0; o < NF; ++o) {
+        if (f0 + o >= p.nf) break;
+        float *are_g = p.a_re + (size_t)(f0 + o) * p.a_stride;
+        float *aim_g = p.a_im + (size_t)(f0 + o) * p.a_stride;
+        const float4 *pl = plane + o * p.plane;
+        for (int e = lane; e < total; e += 32) {
+            const int r = (int)((unsigned)e * inv_c >> 20), c = e - r * ncols;
+            const float4 v = pl[c * ldr + r];
             if (v.x != 0.f || v.y != 0.f) {
-                const size_t off = (size_t)sv * p.b_src_stride + (size_t)f * p.b_stride + p.rows[r0 + r];
-                atomicAdd(p.b_re + off, v.x);
-                atomicAdd(p.b_im + off, v.y);
+                const size_t off = (size_t)s_rows[r] * p.lda + cols[c];
+                atomicAdd(are_g + off, v.x);
+                atomicAdd(aim_g + off, v.y);
             }
         }
-        for (int e = tid; e < nsrc * ncols; e += kAsmThreads) {
-            const int sv = e / ncols, c = e - sv * ncols;
-            const float2 v = rhs2[e];
-            if (v.x != 0.f || v.y != 0.f) {
-                const size_t off = (size_t)sv * p.b_src_stride + (size_t)f * p.b_stride + p.cols[c0 + c];
-                atomicAdd(p.b_re + off, v.x);
-                atomicAdd(p.b_im + off, v.y);
+        for (int e = lane; e < total; e += 32) {
+            const int c = (int)((unsigned)e * inv_r >> 20), r = e - c * nrows;
+            const float4 v = pl[c * ldr + r];
+            if (v.z != 0.f || v.w != 0.f) {
+                const size_t off = (size_t)cols[c] * p.lda + s_rows[r];
+                atomicAdd(are_g + off, v.z);
+                atomicAdd(aim_g + off, v.w);
             }
         }
     }
 }
 
-template <int SYM, bool CK, int MINB>
-cudaError_t launch_regular_sym_t(const AsmArgs &a, dim3 grid, size_t smem, cudaStream_t st) {
-    auto kern = k_regular_sym<SYM, CK, MINB>;
+// ---------------------------------------------------------------------------
+// Right-hand sides: b_i += sum_sigma (int phi_i G) q_sigma over the driven
+// triangles.  A CTA owns a test tile (thread = one of its 32 x 6 quadrature
+// points) x 256 trial triangles, of which it keeps those with Neumann data of
+// any of its sources; per triangle the six points and their images give one
+// complex sum per wavenumber (NF share the geometry), which every source
+// multiplies by its q.  The points' totals are contracted with the basis and
+// added to b per test row at the end.  Sums are nested (triangle, 32
+// triangles, CTA) so that each adds few terms.  Done apart from the matrix:
+// only driven triangles need G, and no 3 x 3 blocks are formed for it.
+// ---------------------------------------------------------------------------
+constexpr int kRhsTrials = 256;   // at most; fewer (p.rhs_block) when that leaves SMs idle
+constexpr int kRhsThreads = kTestTile * 6;
+
+template <int SYM, bool CK, int NF, int NS>
+__global__ void __launch_bounds__(kRhsThreads) k_rhs(const __grid_constant__ AsmArgs p) {
+    constexpr int M = n_images<SYM>(), kBatch = 32;
+    __shared__ float4 s_pt[kBatch * 6];
+    __shared__ float2 s_q[kBatch][NF][NS];   // q times the trial Jacobian
+    __shared__ int s_list[kRhsTrials];
+    __shared__ int s_wcount[kRhsThreads / 32];
+    __shared__ float2 s_red[kRhsThreads];
+    __shared__ __align__(16) unsigned char s_gl[kGatherBytes];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int f0 = p.f_base + blockIdx.z * NF;
+    const int test0 = blockIdx.y * kTestTile, T = p.T;
+    const int tbase = blockIdx.x * p.rhs_block, ntrial = min(p.rhs_block, T - tbase);
+    // driven triangles of this block, in order
+    int count = 0;
+    for (int i0 = 0; i0 < ntrial; i0 += kRhsThreads) {
+        const int i = i0 + tid;
+        bool on = false;
+        if (i < ntrial) {
+            const int orig = p.tri[tbase + i].w;
+            for (int sv = 0; sv < p.n_src; ++sv)
+                for (int f = 0; f < NF; ++f) {
+                    const size_t o = (size_t)sv * p.q_src_stride + (size_t)min(f0 + f, p.nf - 1) * p.q_stride + orig;
+                    on |= p.q_re[o] != 0.f || p.q_im[o] != 0.f;
+                }
+        }
+        const unsigned bits = __ballot_sync(0xffffffffu, on);
+        if (lane == 0) s_wcount[warp] = __popc(bits);
+        __syncthreads();
+        int before = count;
+        for (int w = 0; w < kRhsThreads / 32; ++w) {
+            if (w < warp) before += s_wcount[w];
+            count += s_wcount[w];
+        }
+        if (on) s_list[before + __popc(bits & ((1u << lane) - 1u))] = tbase + i;
+        __syncthreads();
+    }
+    if (count == 0) return;
+    for (int i = tid; i < kGatherBytes / 4; i += kRhsThreads)
+        reinterpret_cast<unsigned *>(s_gl)[i] = p.gather[(size_t)blockIdx.y * (kGatherBytes / 4) + i];
+
+    float k[NF], ki[NF];
+#pragma unroll
+    for (int f = 0; f < NF; ++f) {
+        k[f] = p.k[min(f0 + f, p.nf - 1)];
+        ki[f] = p.ki[min(f0 + f, p.nf - 1)];
+    }
+    const int t = tid / 6, a = tid - 6 * t;
+    const int test = min(test0 + t, T - 1);
+    const float4 x = p.qp[(size_t)test * 6 + a];
+    float2 total[NF][NS];
+#pragma unroll
+    for (int f = 0; f < NF; ++f)
+#pragma unroll
+        for (int sv = 0; sv < NS; ++sv) total[f][sv] = make_float2(0.f, 0.f);
+    for (int l0 = 0; l0 < count; l0 += kBatch) {
+        const int nb = min(kBatch, count - l0);
+        __syncthreads();
+        for (int i = tid; i < nb * 6; i += kRhsThreads) s_pt[i] = p.qp[(size_t)s_list[l0 + i / 6] * 6 + i % 6];
+        for (int i = tid; i < nb * NF * NS; i += kRhsThreads) {
+            const int b = i / (NF * NS), f = i / NS % NF, sv = i % NS;
+            float2 q = make_float2(0.f, 0.f);
+            if (sv < p.n_src) {
+                const int tr = s_list[l0 + b];
+                const size_t o = (size_t)sv * p.q_src_stride + (size_t)min(f0 + f, p.nf - 1) * p.q_stride + p.tri[tr].w;
+                const float jac = p.nrm[tr].w;
+                q = make_float2(p.q_re[o] * jac, p.q_im[o] * jac);
+            }
+            s_q[b][f][sv] = q;
+        }
+        __syncthreads();
+        float2 part[NF][NS];
+#pragma unroll
+        for (int f = 0; f < NF; ++f)
+#pragma unroll
+            for (int sv = 0; sv < NS; ++sv) part[f][sv] = make_float2(0.f, 0.f);
+#pragma unroll 1
+        for (int b = 0; b < nb; ++b) {
+            float gr[NF], gi[NF];
+#pragma unroll
+            for (int f = 0; f < NF; ++f) gr[f] = gi[f] = 0.f;
+#pragma unroll
+            for (int q = 0; q < 6; ++q) {
+                const float4 y = s_pt[b * 6 + q];
+#pragma unroll
+                for (int m = 0; m < M; ++m) {
+                    const int mk = image_mask<SYM>(m);
+                    const float dx = sgn(mk, 0) * y.x - x.x, dy = sgn(mk, 1) * y.y - x.y, dz = sgn(mk, 2) * y.z - x.z;
+                    const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+                    float u = rsqrt_ftz(r2);
+                    u = r2 > 1.0e-14f ? u : 0.0f;
+                    const float r = r2 * u;
+                    float uw = u * qw(q);
+#pragma unroll
+                    for (int f = 0; f < NF; ++f) {
+                        float sn, cs, uf = uw;
+                        __sincosf(r * k[f], &sn, &cs);
+                        if (CK) uf *= __expf(-ki[f] * r);
+                        gr[f] = fmaf(uf, cs, gr[f]);
+                        gi[f] = fmaf(uf, sn, gi[f]);
+                    }
+                }
+            }
+#pragma unroll
+            for (int f = 0; f < NF; ++f)
+#pragma unroll
+                for (int sv = 0; sv < NS; ++sv) {
+                    const float2 q = s_q[b][f][sv];
+                    part[f][sv].x = fmaf(gr[f], q.x, fmaf(-gi[f], q.y, part[f][sv].x));
+                    part[f][sv].y = fmaf(gr[f], q.y, fmaf(gi[f], q.x, part[f][sv].y));
+                }
+        }
+#pragma unroll
+        for (int f = 0; f < NF; ++f)
+#pragma unroll
+            for (int sv = 0; sv < NS; ++sv) {
+                total[f][sv].x += part[f][sv].x;
+                total[f][sv].y += part[f][sv].y;
+            }
+    }
+    const int r0 = p.row_off[blockIdx.y], nrows = p.row_off[blockIdx.y + 1] - r0;
+    const float scale = HBEM_INV4PI * p.rw * p.nrm[test].w;
+#pragma unroll
+    for (int f = 0; f < NF; ++f) {
+        if (f0 + f >= p.nf) break;
+#pragma unroll
+        for (int sv = 0; sv < NS; ++sv) {
+            if (sv >= p.n_src) break;
+            __syncthreads();
+            s_red[tid] = make_float2(total[f][sv].x * scale, total[f][sv].y * scale);
+            __syncthreads();
+            if (tid < nrows) {
+                float vr = 0.f, vi = 0.f;
+                for (int c = s_gl[tid]; c < s_gl[tid + 1]; ++c) {
+                    const int e = s_gl[kGatherList + c], i = e / kTestTile, l = e % kTestTile;
+#pragma unroll
+                    for (int aa = 0; aa < 6; ++aa) {
+                        const float2 v = s_red[l * 6 + aa];
+                        vr = fmaf(c_wa[aa][i], v.x, vr);
+                        vi = fmaf(c_wa[aa][i], v.y, vi);
+                    }
+                }
+                const size_t off = (size_t)sv * p.b_src_stride + (size_t)(f0 + f) * p.b_stride + p.rows[r0 + tid];
+                atomicAdd(p.b_re + off, vr);
+                atomicAdd(p.b_im + off, vi);
+            }
+        }
+    }
+}
+
+template <int SYM, bool CK, int NF, bool ROBIN>
+cudaError_t launch_pairs_t(AsmArgs a, dim3 grid, cudaStream_t st) {
+    auto kern = k_regular_sym<SYM, CK, NF, ROBIN>;
+    const size_t smem = (size_t)kPairWarps * NF * a.plane * sizeof(float4);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    kern<<<grid, kAsmThreads, smem, st>>>(a);
+    kern<<<grid, kPairWarps * 32, smem, st>>>(a);
     return cudaGetLastError();
 }
 
+// Pairs of wavenumbers, then an odd last one alone (Robin walls need G in
+// every pair: one wavenumber at a time).  launches counts the kernels.
+template <int SYM, bool CK>
+cudaError_t launch_pairs(AsmArgs a, int tiles_x, int tiles_y, cudaStream_t st, int &launches) {
+    cudaError_t e = cudaSuccess;
+    // planes of two wavenumbers that would not fit (scattered triangles: up to
+    // 96 x 24 dofs): one at a time
+    const bool fits = (size_t)kPairWarps * 2 * a.plane * sizeof(float4) <= 200 * 1024;
+    const int pairs = a.beta_re || !fits ? 0 : a.nf / 2;
+    if (pairs > 0) {
+        e = launch_pairs_t<SYM, CK, 2, false>(a, dim3(tiles_x, tiles_y, pairs), st);
+        ++launches;
+    }
+    a.f_base = 2 * pairs;
+    if (e == cudaSuccess && a.beta_re) {
+        e = launch_pairs_t<SYM, CK, 1, true>(a, dim3(tiles_x, tiles_y, a.nf), st);
+        ++launches;
+    } else if (e == cudaSuccess && a.f_base < a.nf) {
+        e = launch_pairs_t<SYM, CK, 1, false>(a, dim3(tiles_x, tiles_y, a.nf - a.f_base), st);
+        ++launches;
+    }
+    if (e == cudaSuccess && a.q_re) {
+        a.f_base = 0;
+        const int groups = a.nf > 1 ? (a.nf + 1) / 2 : 1;
+        a.rhs_block = kRhsTrials;
+        while (a.rhs_block > 32 && tiles_y * ((a.T + a.rhs_block - 1) / a.rhs_block) * groups < 6 * 148)
+            a.rhs_block /= 2;
+        const int tx = (a.T + a.rhs_block - 1) / a.rhs_block;
+        const dim3 g2(tx, tiles_y, (a.nf + 1) / 2), g1(tx, tiles_y, a.nf);
+        if (a.n_src > 1) k_rhs<SYM, CK, 2, kMaxSources><<<g2, kRhsThreads, 0, st>>>(a);
+        else if (a.nf > 1) k_rhs<SYM, CK, 2, 1><<<g2, kRhsThreads, 0, st>>>(a);
+        else k_rhs<SYM, CK, 1, 1><<<g1, kRhsThreads, 0, st>>>(a);
+        e = cudaGetLastError();
+        ++launches;
+    }
+    return e;
+}
+
 template <bool CK>
-cudaError_t dispatch_sym_pairs(int sym, const AsmArgs &a, dim3 grid, size_t smem, cudaStream_t st) {
+cudaError_t dispatch_pairs(int sym, const AsmArgs &a, int tiles_x, int tiles_y, cudaStream_t st, int &launches) {
     switch (sym) {
-        case 0: return launch_regular_sym_t<0, CK, 2>(a, grid, smem, st);
-        case 1: return launch_regular_sym_t<1, CK, 2>(a, grid, smem, st);
-        case 2: return launch_regular_sym_t<2, CK, 2>(a, grid, smem, st);
-        case 3: return launch_regular_sym_t<3, CK, 2>(a, grid, smem, st);
-        default: return launch_regular_sym_t<4, CK, 2>(a, grid, smem, st);
+        case 0: return launch_pairs<0, CK>(a, tiles_x, tiles_y, st, launches);
+        case 1: return launch_pairs<1, CK>(a, tiles_x, tiles_y, st, launches);
+        case 2: return launch_pairs<2, CK>(a, tiles_x, tiles_y, st, launches);
+        case 3: return launch_pairs<3, CK>(a, tiles_x, tiles_y, st, launches);
+        default: return launch_pairs<4, CK>(a, tiles_x, tiles_y, st, launches);
     }
 }
 
@@ -1206,8 +1504,6 @@ int launch_regular(Session &s, int n_freq, const float *k_re, const float *k_im,
                    cudaStream_t st, int n_src, long long q_src_stride, long long b_src_stride) {
     if (n_src < 1 || n_src > kMaxSources) return fail(HBEM_ERR_ARG, "assembly: 1 .. 8 sources per pass");
     const size_t smem = (size_t)kAsmFreqs * (s.max_rows * (s.max_cols | 1) + s.max_rows) * sizeof(float2);
-    const size_t smem_sym = (size_t)(s.max_rows * (s.max_cols | 1) + n_src * s.max_rows +
-                                     s.max_cols * (s.max_rows | 1) + n_src * s.max_cols) * sizeof(float2);
     static bool consts_ready[64] = {false};
     if (s.device >= 0 && s.device < 64 && !consts_ready[s.device]) {
         const double QX[6] = {0.4459484909159651, 0.0915762135097710, 0.1081030181680700,
@@ -1231,7 +1527,7 @@ int launch_regular(Session &s, int n_freq, const float *k_re, const float *k_im,
         HBEM_CUDA(cudaMemcpyToSymbol(c_wa2, wa2, sizeof(wa2)));
         consts_ready[s.device] = true;
     }
-    if (smem > 180 * 1024 || smem_sym > 180 * 1024)
+    if (smem > 180 * 1024)
         return fail(HBEM_ERR_ARG, "assembly tile needs too much shared memory (mesh ordering too scattered)");
     for (int f0 = 0; f0 < n_freq; f0 += kMaxFreqPerLaunch) {
         const int nf = std::min(kMaxFreqPerLaunch, n_freq - f0);
@@ -1255,10 +1551,15 @@ int launch_regular(Session &s, int n_freq, const float *k_re, const float *k_im,
         a.nf = nf;
         cudaError_t e;
         if (tuning(HBEM_TUNE_ASM_PAIRS) != 1 || n_src > 1) {
-            // unordered pairs, one wavenumber per grid slice
-            dim3 grid(s.n_trial_tiles, s.n_test_tiles, nf);
-            e = ck ? dispatch_sym_pairs<true>(s.sym, a, grid, smem_sym, st)
-                   : dispatch_sym_pairs<false>(s.sym, a, grid, smem_sym, st);
+            a.chunk_slot = s.d_chunk_slot; a.chunk_off = s.d_chunk_off; a.chunk_cols = s.d_chunk_cols;
+            a.gather = s.d_gather;
+            a.plane = s.max_chunk_cols * (s.max_rows | 1);
+            const int tx = (s.n_triangles + kPairWarps * kChunk - 1) / (kPairWarps * kChunk);
+            int launches = 0;
+            e = ck ? dispatch_pairs<true>(s.sym, a, tx, s.n_test_tiles, st, launches)
+                   : dispatch_pairs<false>(s.sym, a, tx, s.n_test_tiles, st, launches);
+            count_launch(launches - 1);
+            s.launches += launches - 1;
         } else {
             dim3 grid(s.n_trial_tiles, s.n_test_tiles, (nf + kAsmFreqs - 1) / kAsmFreqs);
             e = ck ? dispatch_sym<true>(s.sym, a, grid, smem, st) : dispatch_sym<false>(s.sym, a, grid, smem, st);

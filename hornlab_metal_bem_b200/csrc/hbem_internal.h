@@ -48,6 +48,12 @@ __device__ __forceinline__ void cp_async4(float *dst, const float *src, int src_
 constexpr int kTestTile = 32;    // test triangles per CTA (one per lane)
 constexpr int kTrialTile = 64;   // trial triangles per CTA (split over 8 warps)
 constexpr int kAsmThreads = 256;
+constexpr int kChunk = 8;        // trial triangles per warp of the unordered pair kernel
+// Row lists of a test tile: byte r is the start of row r's entries (and byte
+// r + 1 their end), then from byte kGatherList the entries, vertex * 32 + lane.
+constexpr int kGatherList = 100, kGatherBytes = 200;
+static_assert(kGatherList > 3 * kTestTile && kGatherBytes - kGatherList >= 3 * kTestTile && kGatherBytes % 4 == 0,
+              "row lists");
 
 // Duffy pair record (device), 3 x int4.
 struct DuffyPair {
@@ -67,10 +73,13 @@ struct Session {
     std::vector<float> areas;      // (T,)
     std::vector<float> normals;    // (3, T)
 
-    // spatial order used by the tiled assembly: sorted position -> original id
+    // order used by the tiled assembly: sorted position -> original id, and the
+    // local vertex that takes place l there (3 per position)
     std::vector<int> order;
+    std::vector<unsigned char> perm;
     int n_test_tiles = 0, n_trial_tiles = 0;
     int max_rows = 0, max_cols = 0;  // distinct dofs per test / trial tile
+    int max_chunk_cols = 0;          // distinct dofs per chunk of kChunk trial triangles
 
     // device geometry, sorted order
     float4 *d_qp = nullptr;         // (T, 6) quadrature points (x, y, z, 0)
@@ -82,6 +91,13 @@ struct Session {
     int *d_rows = nullptr;          // concatenated dof lists of test tiles
     int *d_col_off = nullptr;       // (n_trial_tiles + 1)
     int *d_cols = nullptr;
+    // chunks of the unordered pair kernel: slot of each local dof within its
+    // chunk, .w: bit l set when the next triangle of the chunk has another dof
+    // in place l
+    uchar4 *d_chunk_slot = nullptr;
+    int *d_chunk_off = nullptr;     // (n_chunks + 1)
+    int *d_chunk_cols = nullptr;
+    unsigned *d_gather = nullptr;   // (n_test_tiles, kGatherBytes / 4) row lists
 
     // device geometry, original order (Duffy, field, reductions)
     float *d_verts = nullptr;       // (3, V)
@@ -136,6 +152,9 @@ struct Session {
 };
 
 // ---- pieces implemented in separate translation units ---------------------
+// quadrature points of sorted position i (rule point q of the reordered
+// triangle) from the points of the original triangles
+void sorted_points(const Session &s, const std::vector<float4> &qp, std::vector<float4> &sorted);
 int build_duffy_pairs(Session &s, std::vector<DuffyPair> &pairs);
 int image_shared_vertices(const Session &s, int test, int trial, int test_mask, int trial_mask);
 int launch_near(Session &s, int n_freq, const float *k_re, const float *k_im, int n_src, const float *q_re,

@@ -278,8 +278,8 @@ void free_session(Session *s) {
     cudaGetDevice(&prev);
     cudaSetDevice(s->device);
     void *ptrs[] = {s->d_qp, s->d_nrm, s->d_tri, s->d_test_slot, s->d_trial_slot, s->d_row_off, s->d_rows,
-                    s->d_col_off, s->d_cols, s->d_verts, s->d_tris, s->d_l2g, s->d_tags, s->d_areas,
-                    s->d_normals, s->d_fqp, s->d_fnrm, s->d_pairs, s->d_rule, s->d_rule_w, s->d_status, s->ws,
+                    s->d_col_off, s->d_cols, s->d_chunk_slot, s->d_chunk_off, s->d_chunk_cols, s->d_gather,
+                    s->d_verts, s->d_tris, s->d_l2g, s->d_tags, s->d_areas, s->d_normals, s->d_fqp, s->d_fnrm, s->d_pairs, s->d_rule, s->d_rule_w, s->d_status, s->ws,
                     s->d_ap_tris, s->d_ap_local, s->d_sing_bits, s->d_geo64, s->d_near, s->d_subrule};
     for (void *p : ptrs)
         if (p) cudaFree(p);
@@ -296,6 +296,8 @@ const double kQX[6] = {0.4459484909159651, 0.0915762135097710, 0.108103018168070
 const double kQY[6] = {0.4459484909159651, 0.0915762135097700, 0.4459484909159651,
                        0.1081030181680700, 0.0915762135097700, 0.8168475729804580};
 
+int sorted_dof(const Session &s, int i, int l) { return s.l2g[s.order[i] * 3 + s.perm[3 * i + l]]; }
+
 // Build the test/trial tile dof lists of consecutive sorted triangles.
 void tile_plan(const Session &s, int tile, std::vector<int> &off, std::vector<int> &list,
                std::vector<uchar4> &slot, int &max_count) {
@@ -309,7 +311,7 @@ void tile_plan(const Session &s, int tile, std::vector<int> &off, std::vector<in
     for (int t = 0; t < ntiles; ++t) {
         d.clear();
         for (int i = t * tile; i < std::min(T, (t + 1) * tile); ++i)
-            for (int l = 0; l < 3; ++l) d.push_back(s.l2g[s.order[i] * 3 + l]);
+            for (int l = 0; l < 3; ++l) d.push_back(sorted_dof(s, i, l));
         std::sort(d.begin(), d.end());
         d.erase(std::unique(d.begin(), d.end()), d.end());
         off[t] = (int)list.size();
@@ -318,14 +320,158 @@ void tile_plan(const Session &s, int tile, std::vector<int> &off, std::vector<in
         for (int i = t * tile; i < std::min(T, (t + 1) * tile); ++i) {
             unsigned char sl[3];
             for (int l = 0; l < 3; ++l)
-                sl[l] = (unsigned char)(std::lower_bound(d.begin(), d.end(), s.l2g[s.order[i] * 3 + l]) - d.begin());
+                sl[l] = (unsigned char)(std::lower_bound(d.begin(), d.end(), sorted_dof(s, i, l)) - d.begin());
             slot[i] = make_uchar4(sl[0], sl[1], sl[2], 0);
         }
     }
     off[ntiles] = (int)list.size();
 }
 
+
+// Triangle order of the tiled assembly.  Chunks of kChunk and tiles of
+// kTestTile consecutive triangles should touch few distinct dofs, and a
+// triangle should share an edge with the one before it.  Grown greedily over
+// the mesh: the next triangle touches the chunk (else the tile, the previous
+// tile, or comes first in `seed`) and brings the fewest new dofs to the chunk,
+// then to the tile, shares most dofs with the last triangle and leaves the
+// fewest open neighbours.  On the quarter horn of 1950 triangles: 29 dofs a
+// tile and 9.9 a chunk, against 35 and 14 in Morton order alone.
+void cluster_order(const std::vector<int> &l2g, int n_dof, const std::vector<int> &seed, std::vector<int> &order) {
+    const int T = (int)seed.size();
+    std::vector<int> start(n_dof + 1, 0), inc(3 * (size_t)T), rank(T), open(n_dof, 0);
+    for (int v : l2g) { ++start[v + 1]; ++open[v]; }
+    for (int v = 0; v < n_dof; ++v) start[v + 1] += start[v];
+    {
+        std::vector<int> fill(start.begin(), start.end() - 1);
+        for (int t = 0; t < T; ++t)
+            for (int l = 0; l < 3; ++l) inc[fill[l2g[3 * t + l]]++] = t;
+    }
+    for (int i = 0; i < T; ++i) rank[seed[i]] = i;
+    std::vector<char> used(T, 0);
+    // stamps: the chunk, tile and previous tile a dof belongs to last
+    std::vector<int> chunk_of(n_dof, -1), tile_of(n_dof, -1);
+    std::vector<int> chunk, tile, prev_tile;
+    order.clear();
+    order.reserve(T);
+    int next_seed = 0, last = -1;
+    while ((int)order.size() < T) {
+        const int pos = (int)order.size(), ci = pos / kChunk, ti = pos / kTestTile;
+        if (pos % kTestTile == 0) { prev_tile.swap(tile); tile.clear(); }
+        if (pos % kChunk == 0) chunk.clear();
+        int best = -1, key[4] = {0, 0, 0, 0};
+        const std::vector<int> *pools[3] = {&chunk, &tile, &prev_tile};
+        for (int lvl = 0; lvl < 3 && best < 0; ++lvl)
+            for (int v : *pools[lvl])
+                for (int e = start[v]; e < start[v + 1]; ++e) {
+                    const int u = inc[e];
+                    if (used[u]) continue;
+                    int new_c = 0, new_t = 0, with_last = 0, left = 0;
+                    for (int l = 0; l < 3; ++l) {
+                        const int d = l2g[3 * u + l];
+                        new_c += chunk_of[d] != ci;
+                        new_t += tile_of[d] != ti;
+                        left += open[d];
+                        for (int m = 0; m < 3 && last >= 0; ++m) with_last += l2g[3 * last + m] == d;
+                    }
+                    int k[4] = {0, 0, left, rank[u]};
+                    if (lvl == 0) { k[0] = new_c * 8 + new_t; k[1] = -with_last; }
+                    else if (lvl == 1) { k[0] = new_t; k[1] = left; k[2] = -with_last; }
+                    if (best < 0 || std::lexicographical_compare(k, k + 4, key, key + 4)) {
+                        best = u;
+                        std::copy(k, k + 4, key);
+                    }
+                }
+        if (best < 0) {
+            while (used[seed[next_seed]]) ++next_seed;
+            best = seed[next_seed];
+        }
+        used[best] = 1;
+        order.push_back(best);
+        last = best;
+        for (int l = 0; l < 3; ++l) {
+            const int d = l2g[3 * best + l];
+            --open[d];
+            if (chunk_of[d] != ci) { chunk_of[d] = ci; chunk.push_back(d); }
+            if (tile_of[d] != ti) { tile_of[d] = ti; tile.push_back(d); }
+        }
+    }
+}
+
+// Local vertex order of every sorted triangle: within a chunk a dof shared
+// with the triangle before keeps its place, so the pair kernel keeps that
+// column in registers.
+void place_vertices(Session &s) {
+    const int T = s.n_triangles;
+    s.perm.resize(3 * (size_t)T);
+    for (int i = 0; i < T; ++i) {
+        unsigned char *pm = &s.perm[3 * (size_t)i];
+        for (int l = 0; l < 3; ++l) pm[l] = (unsigned char)l;
+        if (i % kChunk == 0) continue;
+        const int *d = &s.l2g[3 * s.order[i]];
+        int place[3] = {-1, -1, -1};
+        bool taken[3] = {false, false, false};
+        for (int l = 0; l < 3; ++l) {
+            const int before = sorted_dof(s, i - 1, l);
+            for (int m = 0; m < 3 && place[l] < 0; ++m)
+                if (!taken[m] && d[m] == before) { place[l] = m; taken[m] = true; }
+        }
+        for (int l = 0; l < 3; ++l)
+            for (int m = 0; m < 3 && place[l] < 0; ++m)
+                if (!taken[m]) { place[l] = m; taken[m] = true; }
+        for (int l = 0; l < 3; ++l) pm[l] = (unsigned char)place[l];
+    }
+}
+
+// .w of the chunk slots: the places whose dof the next triangle of the chunk
+// does not have there
+void mark_last_uses(const Session &s, std::vector<uchar4> &slot) {
+    for (int i = 0; i < s.n_triangles; ++i) {
+        const bool last = i + 1 == s.n_triangles || (i + 1) % kChunk == 0;
+        unsigned char bits = 0;
+        for (int l = 0; l < 3; ++l)
+            if (last || sorted_dof(s, i, l) != sorted_dof(s, i + 1, l)) bits |= (unsigned char)(1 << l);
+        slot[i].w = bits;
+    }
+}
+
+// Row lists of the test tiles (kGatherBytes each)
+std::vector<unsigned> gather_lists(const Session &s, const std::vector<uchar4> &slot, const std::vector<int> &row_off) {
+    const int n = (int)row_off.size() - 1;
+    std::vector<unsigned char> out((size_t)n * kGatherBytes, 0);
+    for (int t = 0; t < n; ++t) {
+        unsigned char *g = &out[(size_t)t * kGatherBytes];
+        int o = 0;
+        for (int r = 0; r < row_off[t + 1] - row_off[t]; ++r) {
+            g[r] = (unsigned char)o;
+            for (int i = t * kTestTile; i < std::min(s.n_triangles, (t + 1) * kTestTile); ++i) {
+                const unsigned char sl[3] = {slot[i].x, slot[i].y, slot[i].z};
+                for (int l = 0; l < 3; ++l)
+                    if (sl[l] == r) g[kGatherList + o++] = (unsigned char)(l * kTestTile + i - t * kTestTile);
+            }
+            g[r + 1] = (unsigned char)o;
+        }
+    }
+    std::vector<unsigned> words(out.size() / 4);
+    std::memcpy(words.data(), out.data(), out.size());
+    return words;
+}
+
 }  // namespace
+
+namespace hbem {
+// The rule's two orbits of three points: point kOwn[orbit][l] is the one
+// nearest to (or farthest from) vertex l, so reordering the vertices permutes
+// the points of each orbit.
+void sorted_points(const Session &s, const std::vector<float4> &qp, std::vector<float4> &sorted) {
+    static const int kOwn[2][3] = {{0, 2, 3}, {1, 4, 5}};
+    sorted.resize((size_t)s.n_triangles * 6);
+    for (int i = 0; i < s.n_triangles; ++i)
+        for (int o = 0; o < 2; ++o)
+            for (int l = 0; l < 3; ++l)
+                sorted[(size_t)i * 6 + kOwn[o][l]] = qp[(size_t)s.order[i] * 6 + kOwn[o][s.perm[3 * (size_t)i + l]]];
+}
+
+}  // namespace hbem
 
 extern "C" int hbem_version(void) { return 100; }
 
@@ -446,8 +592,7 @@ extern "C" int hbem_session_create(const float *vertices_3xv, int n_vertices, co
         nrm[t] = make_float4(s->normals[t], s->normals[T + t], s->normals[2 * T + t], 2.0f * s->areas[t]);
     }
 
-    // Morton order of centroids keeps tiles spatially compact, so a tile of
-    // 32 / 64 triangles touches few distinct dofs.
+    // Morton order of centroids: where cluster_order starts a new patch
     double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
     for (int t = 0; t < T; ++t) {
         double c[3] = {cx[t], cy[t], cz[t]};
@@ -461,22 +606,29 @@ extern "C" int hbem_session_create(const float *vertices_3xv, int n_vertices, co
         uint32_t iz = (uint32_t)std::min(1023.0, (cz[t] - lo[2]) / span * 1023.0);
         code[t] = spread10(ix) | (spread10(iy) << 1) | (spread10(iz) << 2);
     }
-    s->order.resize(T);
-    std::iota(s->order.begin(), s->order.end(), 0);
-    std::stable_sort(s->order.begin(), s->order.end(), [&](int a, int b) { return code[a] < code[b]; });
+    std::vector<int> morton(T);
+    std::iota(morton.begin(), morton.end(), 0);
+    std::stable_sort(morton.begin(), morton.end(), [&](int a, int b) { return code[a] < code[b]; });
+    cluster_order(s->l2g, n_dof, morton, s->order);
+    place_vertices(*s);
 
-    std::vector<float4> sqp((size_t)T * 6), snrm(T);
+    std::vector<float4> sqp, snrm(T);
     std::vector<int4> stri(T);
+    sorted_points(*s, qp, sqp);
     for (int i = 0; i < T; ++i) {
         int t = s->order[i];
-        for (int q = 0; q < 6; ++q) sqp[(size_t)i * 6 + q] = qp[(size_t)t * 6 + q];
         snrm[i] = nrm[t];
-        stri[i] = make_int4(s->l2g[t * 3], s->l2g[t * 3 + 1], s->l2g[t * 3 + 2], t);
+        stri[i] = make_int4(sorted_dof(*s, i, 0), sorted_dof(*s, i, 1), sorted_dof(*s, i, 2), t);
     }
     std::vector<int> row_off, rows, col_off, cols;
     std::vector<uchar4> test_slot, trial_slot;
     tile_plan(*s, kTestTile, row_off, rows, test_slot, s->max_rows);
     tile_plan(*s, kTrialTile, col_off, cols, trial_slot, s->max_cols);
+    std::vector<int> chunk_off, chunk_cols;
+    std::vector<uchar4> chunk_slot;
+    tile_plan(*s, kChunk, chunk_off, chunk_cols, chunk_slot, s->max_chunk_cols);
+    mark_last_uses(*s, chunk_slot);
+    const std::vector<unsigned> gather = gather_lists(*s, test_slot, row_off);
     s->n_test_tiles = (int)row_off.size() - 1;
     s->n_trial_tiles = (int)col_off.size() - 1;
 
@@ -543,6 +695,10 @@ extern "C" int hbem_session_create(const float *vertices_3xv, int n_vertices, co
     U(upload(&s->d_rows, rows.data(), rows.size()));
     U(upload(&s->d_col_off, col_off.data(), col_off.size()));
     U(upload(&s->d_cols, cols.data(), cols.size()));
+    U(upload(&s->d_chunk_slot, chunk_slot.data(), chunk_slot.size()));
+    U(upload(&s->d_chunk_off, chunk_off.data(), chunk_off.size()));
+    U(upload(&s->d_chunk_cols, chunk_cols.data(), chunk_cols.size()));
+    U(upload(&s->d_gather, gather.data(), gather.size()));
     U(upload(&s->d_verts, s->verts.data(), s->verts.size()));
     U(upload(&s->d_tris, s->tris.data(), s->tris.size()));
     U(upload(&s->d_l2g, s->l2g.data(), s->l2g.size()));
