@@ -48,6 +48,9 @@ namespace {
 
 constexpr int kPanelThreads = 512;
 
+// Raised by a bounded device wait that ran out (see wave_fault_check)
+static __device__ int g_wave_fault;
+
 __device__ __forceinline__ float cabs1(float r, float i) { return fabsf(r) + fabsf(i); }
 
 // The panel kernels' complex arithmetic with every rounding fixed (products
@@ -60,6 +63,24 @@ __device__ __forceinline__ void pivot_inverse(float dr, float di, float &ir, flo
     const float den = 1.0f / fmaf(dr, dr, __fmul_rn(di, di));
     ir = __fmul_rn(dr, den);
     ii = __fmul_rn(-di, den);
+}
+// The same without the divide: the hardware reciprocal and one Newton step
+// (at most one unit in the last place off) where |d|^2 is far from the ends of
+// the range, else d scaled by its larger part first.
+__device__ __forceinline__ void pivot_inverse_fast(float dr, float di, float &ir, float &ii) {
+    const float d = fmaf(dr, dr, __fmul_rn(di, di));
+    if (d > 1.0e-30f && d < 1.0e30f) {
+        float den;
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(den) : "f"(d));
+        den = fmaf(den, fmaf(-d, den, 1.0f), den);
+        ir = __fmul_rn(dr, den);
+        ii = __fmul_rn(-di, den);
+    } else {
+        const float s = fmaxf(fabsf(dr), fabsf(di)), a = dr / s, b = di / s;
+        const float den = 1.0f / fmaf(a, a, __fmul_rn(b, b));
+        ir = a * den / s;
+        ii = -b * den / s;
+    }
 }
 __device__ __forceinline__ void cmul_fixed(float xr, float xi, float yr, float yi, float &zr, float &zi) {
     zr = fmaf(xr, yr, -__fmul_rn(xi, yi));
@@ -639,6 +660,530 @@ __global__ void __launch_bounds__(kPanelRowsThreads)
     if (q == 0 && tid == 0 && first_zero && info[b] == 0) info[b] = first_zero;
     // no CTA may exit while another can still read its shared memory
     cluster.sync();
+}
+
+// ---------------------------------------------------------------------------
+// A whole column block (bw <= 64 columns, all rows from k0) factored by one
+// launch: CS CTAs of a cluster hold the panel in shared memory, thread per
+// row (R <= 384 rows a CTA), and work it in sub-blocks of 16 columns that sit
+// in registers.  Rows do not move: each thread tracks the position its row
+// has in the pivoted order (argmax ties go to the lowest position, as
+// icamax on interchanged rows), and the write-back goes to the final
+// positions.
+//
+// Per column one CTA barrier and one exchange: a warp's best row is found by
+// two redux.sync over order-preserving keys and published beside its key
+// (every warp, before it is known to win), so that after the barrier any warp
+// can pick the CTA's winner.  With CS > 1, warp 0 pushes the winner's row and
+// key to every CTA of the cluster with st.async (remote store and transaction
+// count on the receiver's mbarrier in one), and all wait on their own CTA's
+// mbarrier.  Buffers alternate with the column's parity: a CTA sends column
+// j + 2 only after it has every CTA's column j + 1, which is sent after that
+// CTA's threads are done with column j.  Per sub-block: the 16 pivot rows are
+// pulled over DSMEM by every CTA, U12 = L11^-1 A12 is solved there by a thread
+// per column, and each thread updates the rest of its row with its 16
+// multipliers from registers.
+//
+// What bounds it: the latency of a column (2 redux pairs, barrier, exchange,
+// reciprocal, the updates of up to 16 columns).  The kernels it replaces took
+// 2.4-2.7 us a column (one warp reducing between two barriers, rows streamed
+// through shared memory), and three more launches per 16 or 32 columns.
+// ---------------------------------------------------------------------------
+constexpr int kBlkW = 16;            // columns of a sub-block
+constexpr int kBlkMaxRows = 384;     // rows (threads) per CTA
+constexpr int kBlkPitch = 65;        // float2 per panel row
+constexpr int kBlkMaxCta = 16;
+constexpr int kBlkSpin = 1 << 18;
+constexpr int kNoRow = 0x07ffffff;
+
+// Net effect of a block's interchanges on the rows from k0 (offsets from k0):
+// row i < bw ends up with row top[i]; row low[k].x gets row low[k].y < bw.
+struct BlkMoves {
+    int top[64];
+    int2 low[64];
+    int count;
+    int pad[3];
+};
+
+__device__ __forceinline__ uint32_t smem_addr(const void *p) {
+    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
+}
+__device__ __forceinline__ uint32_t cluster_addr(uint32_t local, int rank) {
+    uint32_t a;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(local), "r"(rank));
+    return a;
+}
+__device__ __forceinline__ void st_async16(uint32_t addr, uint32_t mbar, float4 v) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(addr),
+                 "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w), "r"(mbar)
+                 : "memory");
+}
+__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return done;
+}
+
+struct BlkShared {
+    float2 ut[64][kBlkW + 2];                   // pivot rows of the sub-block by column: A12, then U12
+    float2 l[kBlkW][kBlkW];                     // L11: [k][i] = multiplier of pivot row k + 1 + i in column k, else 0
+    float4 slot[2][kBlkMaxRows / 32][kBlkW / 2];   // each warp's best row, by column parity
+    uint4 cand[2][kBlkMaxRows / 32];            // key, position, local row
+    float4 grow[2][kBlkMaxCta][kBlkW / 2];      // each CTA's best row
+    uint4 gcand[2][kBlkMaxCta];
+    unsigned long long bar[2];
+    int loc[kBlkW];                             // CTA << 16 | local row of the sub-block's pivots
+    int pos[kBlkMaxRows];
+};
+
+// Key of |re| + |im| for an unsigned maximum: larger for larger values, 1 for
+// a NaN on the diagonal position (the pivot of a column of NaNs), else 0.
+__device__ __forceinline__ unsigned pivot_key(float2 x, bool diag) {
+    const float a = cabs1(x.x, x.y);
+    return a == a ? __float_as_uint(a) + 2u : (diag ? 1u : 0u);
+}
+
+template <bool CLUSTER>
+__global__ void __launch_bounds__(kBlkMaxRows) k_panel_block(float *a_re, float *a_im, long long lda,
+                                                             long long a_stride, int n, int k0, int bw, int R,
+                                                             int *piv, long long piv_stride, int *info,
+                                                             BlkMoves *moves) {
+    namespace cg = cooperative_groups;
+    extern __shared__ __align__(16) unsigned char s_raw[];
+    BlkShared &S = *reinterpret_cast<BlkShared *>(s_raw);
+    float2 *s_x = reinterpret_cast<float2 *>(s_raw + sizeof(BlkShared));   // [R][kBlkPitch]
+    cg::cluster_group cluster = cg::this_cluster();
+    const int CS = CLUSTER ? (int)cluster.num_blocks() : 1, q = CLUSTER ? (int)cluster.block_rank() : 0;
+    const int b = CLUSTER ? blockIdx.y : blockIdx.x;
+    const int m = n - k0;
+    const int r0 = q * R, nr = min(R, m - r0);   // own rows (may be <= 0 in the last CTA)
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
+    float *gre = a_re + (size_t)b * a_stride + (size_t)k0 * lda + k0;
+    float *gim = a_im + (size_t)b * a_stride + (size_t)k0 * lda + k0;
+    // four columns a thread where every row starts on 16 bytes
+    const bool wide = bw == 64 && (lda & 3) == 0 &&
+                      ((reinterpret_cast<uintptr_t>(gre) | reinterpret_cast<uintptr_t>(gim)) & 15) == 0;
+    if (wide) {
+#pragma unroll 4
+        for (int e = tid; e < nr * 16; e += blockDim.x) {
+            const int r = e >> 4, c = (e & 15) * 4;
+            const size_t o = (size_t)(r0 + r) * lda + c;
+            const float4 re = *reinterpret_cast<const float4 *>(gre + o), im = *reinterpret_cast<const float4 *>(gim + o);
+            float2 *to = s_x + r * kBlkPitch + c;
+            to[0] = make_float2(re.x, im.x);
+            to[1] = make_float2(re.y, im.y);
+            to[2] = make_float2(re.z, im.z);
+            to[3] = make_float2(re.w, im.w);
+        }
+    } else {
+        for (int r = warp; r < nr; r += nw) {
+            const size_t o = (size_t)(r0 + r) * lda;
+            for (int c = lane; c < bw; c += 32) {
+                cp_async4(&s_x[r * kBlkPitch + c].x, gre + o + c, 4);
+                cp_async4(&s_x[r * kBlkPitch + c].y, gim + o + c, 4);
+            }
+        }
+    }
+    for (int e = tid; e < kBlkW * kBlkW; e += blockDim.x) S.l[e / kBlkW][e % kBlkW] = make_float2(0.f, 0.f);
+    if (CLUSTER && tid == 0) {
+        for (int i = 0; i < 2; ++i)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&S.bar[i])));
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    if (CLUSTER) cluster.sync();   // loads done everywhere before any write-back, barriers ready
+    else __syncthreads();
+
+    const bool mine = tid < nr;
+    int pos = mine ? r0 + tid : kNoRow - 1;   // position of this row; positions < current column are done
+    float2 *row = s_x + tid * kBlkPitch;
+    int first_zero = 0;
+    bool dead = false;   // a wait ran out: stop waiting, the results are void
+    int phase = 0;       // bit i: parity of mbarrier i
+#pragma unroll 1
+    for (int q0 = 0; q0 < bw; q0 += kBlkW) {
+        const int w = min(kBlkW, bw - q0);
+        // x[0] is the current column: every column shifts the row left by one
+        float2 x[kBlkW];
+#pragma unroll
+        for (int c = 0; c < kBlkW; ++c) x[c] = mine && c < w ? row[q0 + c] : make_float2(0.f, 0.f);
+        // the warp's best row in column j: key, and position (kNoRow: none)
+        unsigned wk;
+        int wp;
+        auto warp_best = [&](int j) {
+            const bool active = mine && pos >= j;
+            const unsigned key = active ? pivot_key(x[0], pos == j) : 0u;
+            wk = __reduce_max_sync(0xffffffffu, key);
+            wp = __reduce_min_sync(0xffffffffu, active && key == wk ? pos : kNoRow);
+        };
+        // the best of `count` <= 16 candidates (key, position, local row): its index
+        auto best_of = [&](const uint4 *cand, int count) -> int {
+            const uint2 c = lane < count ? *reinterpret_cast<const uint2 *>(cand + lane)
+                                         : make_uint2(0u, (unsigned)kNoRow);
+            const unsigned bk = __reduce_max_sync(0xffffffffu, c.x);
+            return (int)(__reduce_min_sync(0xffffffffu, c.x == bk ? c.y << 4 | (lane & 15) : 0xffffffffu) & 15u);
+        };
+        warp_best(q0);
+#pragma unroll 1
+        for (int j = q0; j < q0 + w; ++j) {
+            const int par = j & 1;
+            if (mine && pos == wp) {
+                float4 *to = S.slot[par][warp];
+#pragma unroll
+                for (int c = 0; c < kBlkW / 2; ++c)
+                    to[c] = make_float4(x[2 * c].x, x[2 * c].y, x[2 * c + 1].x, x[2 * c + 1].y);
+                S.cand[par][warp] = make_uint4(wk, (unsigned)pos, (unsigned)tid, 0u);
+            } else if (lane == 0 && wp == kNoRow) {
+                S.cand[par][warp] = make_uint4(0u, (unsigned)kNoRow, 0u, 0u);   // no active row in this warp
+            }
+            __syncthreads();
+            int best, owner = 0;
+            const float4 *prow;
+            const uint4 *info_of;
+            if (CLUSTER) {
+                const uint32_t bar = smem_addr(&S.bar[par]);
+                if (warp == 0) {
+                    // lanes k < 8 of each half: piece k of the row, lane 8: its key; one CTA a half
+                    best = best_of(S.cand[par], nw);
+                    if (lane == 0)
+                        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
+                                     "r"((kBlkW / 2 + 1) * 16 * CS)
+                                     : "memory");
+                    const int k = lane & 15;
+                    if (k <= kBlkW / 2) {
+                        const float4 v = k < kBlkW / 2 ? S.slot[par][best][k]
+                                                       : *reinterpret_cast<const float4 *>(&S.cand[par][best]);
+                        const uint32_t to = k < kBlkW / 2 ? smem_addr(&S.grow[par][q][k]) : smem_addr(&S.gcand[par][q]);
+                        for (int dst = lane >> 4; dst < CS; dst += 2)
+                            st_async16(cluster_addr(to, dst), cluster_addr(bar, dst), v);
+                    }
+                    __syncwarp();
+                }
+                if (!dead) {
+                    int spins = 0;
+                    while (!mbar_try(bar, (phase >> par) & 1))
+                        if (++spins > kBlkSpin) {
+                            dead = true;
+                            atomicExch(&g_wave_fault, 1);
+                            break;
+                        }
+                }
+                phase ^= 1 << par;
+                owner = best = best_of(S.gcand[par], CS);
+                prow = S.grow[par][best];
+                info_of = &S.gcand[par][best];
+            } else {
+                best = best_of(S.cand[par], nw);
+                prow = S.slot[par][best];
+                info_of = &S.cand[par][best];
+            }
+            float2 u[kBlkW];
+            const uint4 won = *info_of;
+#pragma unroll
+            for (int k = 0; k < kBlkW / 2; ++k) {
+                const float4 v = prow[k];
+                u[2 * k] = make_float2(v.x, v.y);
+                u[2 * k + 1] = make_float2(v.z, v.w);
+            }
+            int p = (int)won.y;
+            if ((unsigned)p >= (unsigned)m) p = j;   // only after a wait that ran out (as the bound on the row)
+            if (tid == 0) {
+                S.loc[j - q0] = owner << 16 | (int)min(won.z, (unsigned)R - 1u);
+                if (q == 0) piv[(size_t)b * piv_stride + k0 + j] = k0 + p;
+            }
+            // interchange: the old row j takes position p
+            if (pos == j) pos = p;
+            else if (pos == p) pos = j;
+            const bool zero = u[0].x == 0.f && u[0].y == 0.f;
+            float ir = 0.f, ii = 0.f;
+            if (zero) {
+                if (first_zero == 0) first_zero = k0 + j + 1;
+#pragma unroll
+                for (int k = 1; k < kBlkW; ++k) u[k] = make_float2(0.f, 0.f);
+            } else {
+                pivot_inverse_fast(u[0].x, u[0].y, ir, ii);
+            }
+            if (pos == j) {   // this row is done: its part of U
+#pragma unroll
+                for (int k = 0; k < kBlkW; ++k)
+                    if (k < q0 + w - j) row[j + k] = x[k];
+            }
+            float lr, li;
+            cmul_fixed(x[0].x, x[0].y, ir, ii, lr, li);
+            if (mine && pos > j) row[j] = make_float2(lr, li);
+            // rows that are done shift along, unused
+            auto eliminate = [&](int k) {
+                x[k - 1].x = fmaf(-lr, u[k].x, fmaf(li, u[k].y, x[k].x));
+                x[k - 1].y = fmaf(-lr, u[k].y, fmaf(-li, u[k].x, x[k].y));
+            };
+            eliminate(1);
+            warp_best(j + 1);
+#pragma unroll
+            for (int k = 2; k < kBlkW; ++k) eliminate(k);
+            x[kBlkW - 1] = make_float2(0.f, 0.f);
+        }
+        const int c1 = q0 + w;   // first column right of the sub-block (w = 16 unless it is the last)
+        if (c1 >= bw) break;
+        // pivot rows from their owners: multipliers to l, columns right of the sub-block to ut
+        if (CLUSTER) cluster.sync();
+        else __syncthreads();
+        for (int e = tid; e < kBlkW * 64; e += blockDim.x) {
+            const int i = e >> 6, col = e & 63, k = col - q0;
+            if (k < 0 || col >= bw || (k >= i && k < kBlkW)) continue;
+            const int loc = S.loc[i];
+            const float2 *src = s_x + (loc & 0xffff) * kBlkPitch + col;
+            const float2 v = CLUSTER ? *cluster.map_shared_rank(src, loc >> 16) : *src;
+            if (k < kBlkW) S.l[k][i - k - 1] = v;
+            else S.ut[col][i] = v;
+        }
+        if (CLUSTER) asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+        __syncthreads();
+        // U12 = L11^-1 A12, a thread per column, its entries shifting as the rows above
+        if (tid < bw - c1) {
+            float2 *col = S.ut[c1 + tid];
+            float2 y[kBlkW];
+#pragma unroll
+            for (int i = 0; i < kBlkW; ++i) y[i] = col[i];
+#pragma unroll 1
+            for (int k = 0; k < kBlkW; ++k) {
+                const float2 v = y[0];
+                col[k] = v;
+                const float4 *l4 = reinterpret_cast<const float4 *>(S.l[k]);
+#pragma unroll
+                for (int i = 0; i < kBlkW; i += 2) {
+                    const float4 l = l4[i / 2];
+                    if (i + 1 < kBlkW) {
+                        y[i].x = fmaf(-l.x, v.x, fmaf(l.y, v.y, y[i + 1].x));
+                        y[i].y = fmaf(-l.x, v.y, fmaf(-l.y, v.x, y[i + 1].y));
+                    }
+                    if (i + 2 < kBlkW) {
+                        y[i + 1].x = fmaf(-l.z, v.x, fmaf(l.w, v.y, y[i + 2].x));
+                        y[i + 1].y = fmaf(-l.z, v.y, fmaf(-l.w, v.x, y[i + 2].y));
+                    }
+                }
+                y[kBlkW - 1] = make_float2(0.f, 0.f);
+            }
+        }
+        __syncthreads();
+        // every CTA has its copy of the pivot rows: they may be overwritten
+        if (CLUSTER) asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+        if (mine && pos >= c1) {
+#pragma unroll
+            for (int k = 0; k < kBlkW; ++k) x[k] = row[q0 + k];
+            // four columns at a time: independent chains of FMAs
+            int col = c1;
+            for (; col + 4 <= bw; col += 4) {
+                float2 a[4];
+#pragma unroll
+                for (int t = 0; t < 4; ++t) a[t] = row[col + t];
+#pragma unroll
+                for (int k = 0; k < kBlkW; k += 2)
+#pragma unroll
+                    for (int t = 0; t < 4; ++t) {
+                        const float4 v = *reinterpret_cast<const float4 *>(&S.ut[col + t][k]);
+                        a[t].x = fmaf(-x[k].x, v.x, fmaf(x[k].y, v.y, a[t].x));
+                        a[t].y = fmaf(-x[k].x, v.y, fmaf(-x[k].y, v.x, a[t].y));
+                        a[t].x = fmaf(-x[k + 1].x, v.z, fmaf(x[k + 1].y, v.w, a[t].x));
+                        a[t].y = fmaf(-x[k + 1].x, v.w, fmaf(-x[k + 1].y, v.z, a[t].y));
+                    }
+#pragma unroll
+                for (int t = 0; t < 4; ++t) row[col + t] = a[t];
+            }
+#pragma unroll 1
+            for (; col < bw; ++col) {
+                float2 a = row[col];
+#pragma unroll
+                for (int k = 0; k < kBlkW; ++k) {
+                    const float2 v = S.ut[col][k];
+                    a.x = fmaf(-x[k].x, v.x, fmaf(x[k].y, v.y, a.x));
+                    a.y = fmaf(-x[k].x, v.y, fmaf(-x[k].y, v.x, a.y));
+                }
+                row[col] = a;
+            }
+        } else if (mine && pos >= q0) {
+            for (int col = c1; col < bw; ++col) row[col] = S.ut[col][pos - q0];
+        }
+    }
+    if (mine) {
+        S.pos[tid] = pos;
+        // the interchanges' net effect, for the columns outside the block
+        BlkMoves &mv = moves[b];
+        if (pos < bw) {
+            mv.top[pos] = r0 + tid;
+        } else if (pos != r0 + tid) {
+            const int i = atomicAdd(&mv.count, 1);
+            if (i < 64) mv.low[i] = make_int2(pos, r0 + tid);   // at most bw unless a wait ran out
+        }
+    }
+    __syncthreads();
+    if (wide) {
+#pragma unroll 4
+        for (int e = tid; e < nr * 16; e += blockDim.x) {
+            const int r = e >> 4, c = (e & 15) * 4;
+            const size_t o = (size_t)S.pos[r] * lda + c;
+            const float2 *v = s_x + r * kBlkPitch + c;
+            *reinterpret_cast<float4 *>(gre + o) = make_float4(v[0].x, v[1].x, v[2].x, v[3].x);
+            *reinterpret_cast<float4 *>(gim + o) = make_float4(v[0].y, v[1].y, v[2].y, v[3].y);
+        }
+    } else {
+        for (int r = warp; r < nr; r += nw) {
+            const size_t o = (size_t)S.pos[r] * lda;
+            for (int c = lane; c < bw; c += 32) {
+                const float2 v = s_x[r * kBlkPitch + c];
+                gre[o + c] = v.x;
+                gim[o + c] = v.y;
+            }
+        }
+    }
+    if (q == 0 && tid == 0 && first_zero && info[b] == 0) info[b] = first_zero;
+    if (CLUSTER) cluster.sync();   // no CTA may exit while another can still read or write its shared memory
+}
+
+// Row moves of a block factored by k_panel_block and U12 = L11^-1 A12, for up
+// to kMoveCols columns per CTA of [col_lo, col_hi) minus [ex_lo, ex_lo + ex_w);
+// columns from trsm_lo on are solved.  Every row is read once from where the
+// interchanges' net effect takes it (no replay of the sequence): the bw top
+// rows into shared memory, the rows that go below straight to registers, and
+// after the barrier to their places.  The solve goes in blocks of 8 rows: warp
+// 0 (a lane per column) takes the diagonal triangle with the column in
+// registers, then all warps update the rows below.
+//
+// What bounds it: latency (the list, the rows, 8 diagonal blocks).  The replay
+// of the sequence in shared memory by k_swap_trsm and its 16-row triangles of
+// straight-line code took 25-32 us a launch at n = 1043, this 6-8 us.
+constexpr int kMoveCols = 32;
+constexpr int kMoveThreads = 256;
+
+__global__ void __launch_bounds__(kMoveThreads) k_move_solve(float *a_re, float *a_im, long long lda,
+                                                             long long a_stride, int n, int k0, int bw, int col_lo,
+                                                             int col_hi, int ex_lo, int ex_w, int trsm_lo,
+                                                             const BlkMoves *moves) {
+    constexpr int NW = kMoveThreads / 32, XP = kMoveCols;
+    __shared__ float2 s_x[64 * XP];
+    // L11 in blocks of 8 columns, rows from the block's first: row r of block i at i (60 - 4 i) + r
+    __shared__ __align__(16) float2 s_l[288][8];
+    __shared__ int s_top[64];
+    __shared__ int2 s_low[64];
+    const int b = blockIdx.y;
+    float *are = a_re + (size_t)b * a_stride + (size_t)k0 * lda, *aim = a_im + (size_t)b * a_stride + (size_t)k0 * lda;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const BlkMoves &mv = moves[b];
+    const int count = min(mv.count, 64);
+    // (bounds that only matter after a panel's wait ran out)
+    auto row_of = [&](int r) { return min(max(r, 0), n - k0 - 1); };
+    if (tid < bw) s_top[tid] = row_of(mv.top[tid]);
+    if (tid >= 64 && tid - 64 < count) {
+        const int2 v = mv.low[tid - 64];
+        s_low[tid - 64] = make_int2(row_of(v.x), row_of(v.y));
+    }
+    const int ncols = min(kMoveCols, col_hi - col_lo - ex_w - (int)blockIdx.x * kMoveCols);
+    int col = col_lo + blockIdx.x * kMoveCols + lane;
+    if (col >= ex_lo) col += ex_w;
+    const bool on = lane < ncols;
+    const bool solve = on && col >= trsm_lo;
+    const bool any_solve = __syncthreads_or(solve);
+    if (any_solve) {   // strictly lower triangle of L11, zeros above
+#pragma unroll 8
+        for (int e = tid; e < 64 * 64; e += kMoveThreads) {
+            const int r = e >> 6, c = e & 63, i = c >> 3;
+            float2 v = make_float2(0.f, 0.f);
+            if (r < bw && c < r) v = make_float2(are[(size_t)r * lda + k0 + c], aim[(size_t)r * lda + k0 + c]);
+            if (r >= 8 * i) s_l[i * (60 - 4 * i) + r][c & 7] = v;
+        }
+    }
+    float2 below[64 / NW];
+#pragma unroll
+    for (int i = 0; i < 64 / NW; ++i) {
+        const int k = warp + i * NW;
+        below[i] = make_float2(0.f, 0.f);
+        if (on && k < count) {
+            const size_t o = (size_t)s_low[k].y * lda + col;
+            below[i] = make_float2(are[o], aim[o]);
+        }
+    }
+    float2 x[64 / NW];
+#pragma unroll
+    for (int i = 0; i < 64 / NW; ++i) {
+        const int r = warp + i * NW;
+        x[i] = make_float2(0.f, 0.f);
+        if (on && r < bw) {
+            const size_t o = (size_t)s_top[r] * lda + col;
+            x[i] = make_float2(are[o], aim[o]);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 64 / NW; ++i) s_x[(warp + i * NW) * XP + lane] = x[i];
+    __syncthreads();   // every row is read
+#pragma unroll
+    for (int i = 0; i < 64 / NW; ++i) {
+        const int k = warp + i * NW;
+        if (on && k < count) {
+            const size_t o = (size_t)s_low[k].x * lda + col;
+            are[o] = below[i].x;
+            aim[o] = below[i].y;
+        }
+    }
+    if (any_solve) {
+#pragma unroll 1
+        for (int q0 = 0; q0 < bw; q0 += 8) {
+            const int i0 = q0 >> 3;
+            const float2 (*lb)[8] = s_l + i0 * (60 - 4 * i0);   // row r of L11's columns q0 .. q0+7
+            if (warp == 0 && solve) {
+                float2 y[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) y[i] = s_x[(q0 + i) * XP + lane];
+#pragma unroll
+                for (int k = 0; k < 7; ++k)
+#pragma unroll
+                    for (int i = k + 1; i < 8; ++i) {
+                        const float2 l = lb[q0 + i][k];
+                        y[i].x = fmaf(-l.x, y[k].x, fmaf(l.y, y[k].y, y[i].x));
+                        y[i].y = fmaf(-l.x, y[k].y, fmaf(-l.y, y[k].x, y[i].y));
+                    }
+#pragma unroll
+                for (int i = 1; i < 8; ++i) s_x[(q0 + i) * XP + lane] = y[i];
+            }
+            __syncthreads();
+            if (solve && q0 + 8 < bw) {
+                float2 y[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) y[i] = s_x[(q0 + i) * XP + lane];
+#pragma unroll 2
+                for (int r = q0 + 8 + warp; r < bw; r += NW) {
+                    float2 v = s_x[r * XP + lane];
+                    const float4 *l4 = reinterpret_cast<const float4 *>(lb[r]);
+#pragma unroll
+                    for (int k = 0; k < 8; k += 2) {
+                        const float4 l = l4[k / 2];
+                        v.x = fmaf(-l.x, y[k].x, fmaf(l.y, y[k].y, v.x));
+                        v.y = fmaf(-l.x, y[k].y, fmaf(-l.y, y[k].x, v.y));
+                        v.x = fmaf(-l.z, y[k + 1].x, fmaf(l.w, y[k + 1].y, v.x));
+                        v.y = fmaf(-l.z, y[k + 1].y, fmaf(-l.w, y[k + 1].x, v.y));
+                    }
+                    s_x[r * XP + lane] = v;
+                }
+            }
+            __syncthreads();
+        }
+    }
+    if (on) {
+#pragma unroll
+        for (int i = 0; i < 64 / NW; ++i) {
+            const int r = warp + i * NW;
+            if (r < bw) {
+                const float2 v = s_x[r * XP + lane];
+                are[(size_t)r * lda + col] = v.x;
+                aim[(size_t)r * lda + col] = v.y;
+            }
+        }
+    }
 }
 
 // Row swaps + forward substitution for a column range, staged in shared
@@ -1334,8 +1879,6 @@ struct WaveCtl {
     int pad;
 };
 
-static __device__ int g_wave_fault;
-
 // A non-zero status word of a factorisation's tensor-core update raises the
 // fault word as well.
 __global__ void k_fold_status(const int *status) {
@@ -1988,6 +2531,78 @@ int launch_panel_cluster(float *a_re, float *a_im, long long lda, long long a_st
     return launch_panel_cluster_t<16>(a_re, a_im, lda, a_stride, n, c, w, piv, piv_stride, info, batch, R, smem, st);
 }
 
+// CTAs per matrix of the block panel kernel for m rows, 0 when the panel does
+// not fit a cluster.
+int panel_block_ctas(int m, int batch) {
+    const int least = (m + kBlkMaxRows - 1) / kBlkMaxRows;
+    if (least > kBlkMaxCta) return 0;
+    return least;
+}
+
+int launch_panel_block(float *a_re, float *a_im, long long lda, long long a_stride, int n, int c, int w, int *piv,
+                       long long piv_stride, int *info, int batch, int cs, BlkMoves *moves, cudaStream_t st) {
+    const int m = n - c;
+    const int R = ((m + cs - 1) / cs + 31) & ~31;
+    const size_t smem = sizeof(BlkShared) + (size_t)R * kBlkPitch * sizeof(float2);
+    if (cs == 1) {
+        const int rc = func_opt_in((const void *)k_panel_block<false>, 227 * 1024);
+        if (rc != HBEM_OK) return rc;
+        k_panel_block<false><<<batch, R, smem, st>>>(a_re, a_im, lda, a_stride, n, c, w, R, piv, piv_stride, info,
+                                                     moves);
+        HBEM_LAUNCH_CHECK("k_panel_block");
+        return HBEM_OK;
+    }
+    {
+        const int rc = func_opt_in((const void *)k_panel_block<true>, 227 * 1024, true);
+        if (rc != HBEM_OK) return rc;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(cs, batch);
+    cfg.blockDim = dim3(R);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = cs;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    HBEM_CUDA(cudaLaunchKernelEx(&cfg, k_panel_block<true>, a_re, a_im, lda, a_stride, n, c, w, R, piv, piv_stride,
+                                 info, moves));
+    HBEM_LAUNCH_CHECK("k_panel_block");
+    return HBEM_OK;
+}
+
+// Whether a cluster of cs full-size panel CTAs can be resident (sizes above 8
+// are not portable, and those that are no power of two need not divide a GPC)
+bool panel_block_fits(int cs) {
+    if (cs == 1) return true;
+    static std::atomic<int> cached[64][kBlkMaxCta + 1];   // 0 unknown, 1 yes, 2 no; a race repeats the query
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
+    if (const int c = cached[dev][cs].load()) return c == 1;
+    int clusters = 0;
+    bool ok = false;
+    if (func_opt_in((const void *)k_panel_block<true>, 227 * 1024, true) == HBEM_OK) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(cs, 1);
+        cfg.blockDim = dim3(kBlkMaxRows);
+        cfg.dynamicSmemBytes = sizeof(BlkShared) + (size_t)kBlkMaxRows * kBlkPitch * sizeof(float2);
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = cs;
+        at[0].val.clusterDim.y = 1;
+        at[0].val.clusterDim.z = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        ok = cudaOccupancyMaxActiveClusters(&clusters, k_panel_block<true>, &cfg) == cudaSuccess && clusters > 0;
+    }
+    cudaGetLastError();   // a refused query leaves no sticky error
+    cached[dev][cs].store(ok ? 1 : 2);
+    return ok;
+}
+
 // Look-ahead streams of one caller stream: the factorisation chain runs on a
 // high-priority stream, the bulk of each trailing update on a low-priority
 // one; both fork from and join back into the caller's stream (so a CUDA
@@ -2095,6 +2710,26 @@ int lu_factor(int n, int batch, float *a_re, float *a_im, long long lda, long lo
             return rc;
         }
     }
+    // Whole 64-column blocks by k_panel_block, where the caller refines the
+    // solution (n = 1043: one matrix 3.89 -> 2.13 ms, 40 matrices 5.97 -> 4.80
+    // ms; 4168 x 6 mixed 25.9 -> 17.8 ms).  HBEM_PREC_PLAIN keeps the 16 to
+    // 64-column panels and their roundings: without refinement another order
+    // of the same sums moves the solution of an ill-conditioned system as far
+    // as its error (a shape gradient at n = 2082 by 2e-4).
+    const bool block_panels = precision != HBEM_PREC_PLAIN && tuning(HBEM_TUNE_LU_PANEL) == 0;
+    // net row moves of the blocks k_panel_block factors
+    BlkMoves *moves = nullptr, *block_moves = nullptr;   // all blocks', and the current block's (NULL: from piv)
+    if (block_panels) {
+        const size_t count = (size_t)((n + 63) / 64) * batch;
+        cudaError_t e = cudaMallocAsync((void **)&moves, count * sizeof(BlkMoves), st);
+        if (e == cudaSuccess) e = cudaMemset2DAsync(&moves->count, sizeof(BlkMoves), 0, sizeof(int), count, st);
+        if (e != cudaSuccess) {
+            if (moves) cudaFreeAsync(moves, st);
+            tc_workspace_destroy(tc, st);
+            if (status) cudaFreeAsync(status, st);
+            return cuda_fail(e, "hbem_lu_factor: row moves");
+        }
+    }
     LookaheadStreams *la = nullptr;
     if (n > 2 * NB && tuning(HBEM_TUNE_LU_LOOKAHEAD) != 1) {
         int rc = lookahead_streams(st, &la);
@@ -2115,6 +2750,7 @@ int lu_factor(int n, int batch, float *a_re, float *a_im, long long lda, long lo
             cudaStreamWaitEvent(st, la->join_bulk, 0);
         }
         tc_workspace_destroy(tc, st);
+        if (moves) cudaFreeAsync(moves, st);
         if (status) {
             // nothing waits for the host here (the caller's next launches
             // queue behind the factorisation, and a graph capture may be
@@ -2164,6 +2800,12 @@ int lu_factor(int n, int batch, float *a_re, float *a_im, long long lda, long lo
             return false;
         return true;
     };
+    // CTAs of the block panel kernel for a panel of that many rows (0: not this kernel)
+    auto block_ctas = [&](int rows) -> int {
+        if (!block_panels) return 0;
+        const int ctas = panel_block_ctas(rows, batch);
+        return ctas > 0 && panel_block_fits(ctas) ? ctas : 0;
+    };
     HBEM_CUDA(cudaFuncSetAttribute(k_swap_trsm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSwapSmem));
     const int cmax = panel_cluster_max(smem_cap);
     // Row swaps of block [b0, b0 + bw) on the columns [lo, hi) minus
@@ -2175,6 +2817,12 @@ int lu_factor(int n, int batch, float *a_re, float *a_im, long long lda, long lo
     auto swap_trsm = [&](int b0, int bw, int lo, int hi, int ex, int exw, int t_lo, int t_hi,
                          cudaStream_t s) -> int {
         if (hi - lo - exw <= 0) return HBEM_OK;
+        if (block_moves) {
+            const dim3 g((hi - lo - exw + kMoveCols - 1) / kMoveCols, batch);
+            k_move_solve<<<g, kMoveThreads, 0, s>>>(a_re, a_im, lda, a_stride, n, b0, bw, lo, hi, ex, exw, b0 + bw,
+                                                    block_moves);
+            return launched("k_move_solve");
+        }
         dim3 grid((hi - lo - exw + kSwapCols - 1) / kSwapCols, batch);
         k_swap_trsm<<<grid, kSwapThreads, kSwapSmem, s>>>(a_re, a_im, lda, a_stride, b0, std::min(bw, 64), lo, hi, ex,
                                                           exw, b0 + bw, piv, piv_stride);
@@ -2204,15 +2852,23 @@ int lu_factor(int n, int batch, float *a_re, float *a_im, long long lda, long lo
         int nbi;
         if (want == 16) nbi = 16;
         else if (want == 32) nbi = rows <= 8 * (smem_cap / (33 * 8)) ? 32 : 16;
+        else if (block_ctas((int)rows) > 0) nbi = 64;
         else if (rows * 65 * 8 <= smem_cap || (want == 64 && rows <= 8 * (smem_cap / (65 * 8)))) nbi = 64;
         else if (rows * 33 * 8 <= smem_cap) nbi = 32;
         else if (rows * 17 * 8 <= smem_cap) nbi = 16;
         else nbi = rows <= 8 * (smem_cap / (33 * 8)) ? 32 : 16;
+        block_moves = nullptr;
         for (int c = b0; c < b0 + bw; c += nbi) {
             const int w = std::min(nbi, b0 + bw - c);
             const size_t psmem = (size_t)(n - c) * (w + 1) * 8;
             int rc = HBEM_OK;
-            if (panel_in_registers(c, w)) {
+            const int cs_blk = block_ctas(n - c);
+            if (cs_blk > 0) {
+                BlkMoves *mv = moves + (size_t)(c / 64) * batch;
+                rc = launch_panel_block(a_re, a_im, lda, a_stride, n, c, w, piv, piv_stride, info, batch, cs_blk, mv,
+                                        cs);
+                if (w == bw) block_moves = mv;
+            } else if (panel_in_registers(c, w)) {
                 rc = launched("k_panel_reg");
             } else if (psmem <= smem_cap) {
                 k_panel_rows<<<batch, kPanelRowsThreads, psmem, cs>>>(a_re, a_im, lda, a_stride, n, c, w, piv, piv_stride,
