@@ -415,9 +415,10 @@ __global__ void __launch_bounds__(kAsmThreads, MINB) k_regular(const __grid_cons
 //   F = e^{ikr} (ik - 1/r) / r^2,  d = My - x,  r = |d| = |Mx - y|
 // (M is an involution and an isometry).  So each unordered pair {tau, sigma}
 // (sorted index tau <= sigma) is evaluated once and adds A[tau dofs][sigma
-// dofs] and A[sigma dofs][tau dofs].  d . M n_sigma is the same for every
-// point of the flat triangle M sigma, so it is formed once per test point and
-// image, scaled by both Jacobians.
+// dofs] and A[sigma dofs][tau dofs].  The Jacobians scale 1/r^2.  d . M n_sigma
+// is taken per sample although it is the same for all points of a flat
+// triangle: formed once per test point it carries one point's rounding into
+// all six, 4e-7 of A (and 1e-4 of a shape gradient) for 4 % of the time.
 //
 // Split.  A warp owns 32 test triangles (one per lane) x a chunk of 8 trial
 // triangles (warp-uniform); 4 such warps share a CTA's test tile.  NF = 2
@@ -439,9 +440,9 @@ __global__ void __launch_bounds__(kAsmThreads, MINB) k_regular(const __grid_cons
 // Bound: issue (a packed instruction takes two slots of the FP32 pipe; 82 % of
 // them busy with one image), with four images the MUFU pipe as well (1 rsqrt
 // + 2 NF per sample: 62 %).  Regular assembly with right-hand sides, 40
-// wavenumbers: quarter horn (1950 triangles, 4 images) 15.8 -> 9.6 ms, half
-// horn (3664, 2 images) 40.0 -> 21.1 ms; full horn (8332, 6 wavenumbers)
-// 26.0 -> 11.7 ms; sphere with every face driven (1280, 8) 2.33 -> 0.72 ms.
+// wavenumbers: quarter horn (1950 triangles, 4 images) 15.8 -> 9.8 ms, half
+// horn (3664, 2 images) 40.0 -> 21.9 ms; full horn (8332, 6 wavenumbers)
+// 26.0 -> 12.2 ms; sphere with every face driven (1280, 8) 2.33 -> 0.74 ms.
 // Two CTAs an SM with 255 registers each were 2-8 % slower than three with 168.
 // ---------------------------------------------------------------------------
 constexpr int kPairWarps = 4;
@@ -471,35 +472,23 @@ struct PairAcc {
     float2 r[NF][9], i[NF][9];
 };
 
-// One unordered pair accumulated into acc.  hn is the scaled trial normal
-// (times -1), tn the scaled test normal; both zero for a lane whose pair does
-// not count.  drop0: the pair of a triangle with itself (its own plane: no
-// double layer, and no transposed block).
+// One unordered pair accumulated into acc.  (hx, hy, hz) is minus the trial
+// normal, (tnx, tny, tnz) the test normal (zero for the pair of a triangle
+// with itself, which has no transposed block); scale zero for a lane whose
+// pair does not count.
 template <int SYM, bool CK, int NF, bool ROBIN>
 __device__ __forceinline__ void pair_accumulate(const float4 *__restrict__ tq, const float4 *__restrict__ sp, float hx,
-                                                float hy, float hz, float tnx, float tny, float tnz, bool self,
+                                                float hy, float hz, float tnx, float tny, float tnz, float scale,
                                                 float2 k2, float2 nk2, float2 ki2, PairAcc<NF> &acc, float (&sfr)[3],
                                                 float (&sfi)[3], float (&str_)[3], float (&sti)[3]) {
     constexpr int M = n_images<SYM>();
     // The test-point loop stays rolled (test point from shared memory, weights
     // from constant memory) so the kernel body fits the instruction cache; the
     // trial-point loop is unrolled with the image samples.  Two test points at
-    // a time pay with two images only (half horn of 3664 triangles x 40
-    // wavenumbers 21.9 -> 21.1 ms; one image 11.7 -> 12.1 ms).
+    // a time pay with two images only (4 %; one image is 3 % slower so).
 #pragma unroll(M == 2 ? 2 : 1)
     for (int a = 0; a < 6; ++a) {
         const float4 x = tq[a * kTestTile];
-        float hp[M];   // -scale (M y - x) . M n_sigma, the same for every y of the triangle
-        {
-            const float4 y = sp[0];
-#pragma unroll
-            for (int m = 0; m < M; ++m) {
-                const int mk = image_mask<SYM>(m);
-                hp[m] = fmaf(sgn(mk, 0) * y.x - x.x, sgn(mk, 0) * hx,
-                             fmaf(sgn(mk, 1) * y.y - x.y, sgn(mk, 1) * hy, (sgn(mk, 2) * y.z - x.z) * (sgn(mk, 2) * hz)));
-            }
-            if (self) hp[0] = 0.f;
-        }
         float2 er[NF][3], ei[NF][3];   // NF = 2: [0] forward, [1] transposed
         float hre = 0.f, him = 0.f, g2r[3], g2i[3];
 #pragma unroll
@@ -523,9 +512,9 @@ __device__ __forceinline__ void pair_accumulate(const float4 *__restrict__ tq, c
                 // keeps the coincident point finite (its factors are 0)
                 const float r2 = fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, 1.0e-30f)));
                 const float u = rsqrt_ftz(r2);
-                const float r = r2 * u, u2 = u * u;
-                const float hh = hp[m] * u2;
-                const float tt = fmaf(dx, tnx, fmaf(dy, tny, dz * tnz)) * u2;
+                const float r = r2 * u, us = u * u * scale;
+                const float hh = fmaf(dx, sgn(mk, 0) * hx, fmaf(dy, sgn(mk, 1) * hy, dz * (sgn(mk, 2) * hz))) * us;
+                const float tt = fmaf(dx, tnx, fmaf(dy, tny, dz * tnz)) * us;
                 // P + i Q = -e^{ikr} (ik - 1/r), with k = k + i ki
                 if constexpr (NF == 2) {
                     const float2 ph = __fmul2_rn(dup2(r), k2);
@@ -540,7 +529,7 @@ __device__ __forceinline__ void pair_accumulate(const float4 *__restrict__ tq, c
                         fre = __fadd2_rn(fre, ki2);
                     }
                     const float2 P = __ffma2_rn(cs, fre, __fmul2_rn(sn, k2));
-                    const float2 Q = __ffma2_rn(sn, fre, __fmul2_rn(cs, nk2));
+                    const float2 Q = __ffma2_rn(cs, nk2, __fmul2_rn(sn, fre));
                     const float2 h2 = dup2(hh), t2 = dup2(tt);
                     dr[0] = __ffma2_rn(P, h2, dr[0]);
                     di[0] = __ffma2_rn(Q, h2, di[0]);
@@ -555,7 +544,7 @@ __device__ __forceinline__ void pair_accumulate(const float4 *__restrict__ tq, c
                         cs *= damp;
                         fre += ki2.x;
                     }
-                    const float P = fmaf(cs, fre, sn * k2.x), Q = fmaf(sn, fre, cs * nk2.x);
+                    const float P = fmaf(cs, fre, sn * k2.x), Q = fmaf(cs, nk2.x, sn * fre);
                     const float2 h2 = make_float2(hh, tt);
                     dr[0] = __ffma2_rn(h2, dup2(P), dr[0]);
                     di[0] = __ffma2_rn(h2, dup2(Q), di[0]);
@@ -714,9 +703,9 @@ __global__ void __launch_bounds__(kPairWarps * 32, NF == 2 ? 3 : 4) k_regular_sy
         const float scale = live && sigma >= test0 + lane ? tscale * nj.w : 0.f;
         const float ts = self ? 0.f : scale;
         float sfr[3] = {0.f, 0.f, 0.f}, sfi[3] = {0.f, 0.f, 0.f}, str_[3] = {0.f, 0.f, 0.f}, sti[3] = {0.f, 0.f, 0.f};
-        pair_accumulate<SYM, CK, NF, ROBIN>(&s_tq[lane], &s_qp[warp][jj * 6], -scale * nj.x, -scale * nj.y,
-                                            -scale * nj.z, ts * tn.x, ts * tn.y, ts * tn.z, self, k2, nk2, ki2, acc,
-                                            sfr, sfi, str_, sti);
+        pair_accumulate<SYM, CK, NF, ROBIN>(&s_tq[lane], &s_qp[warp][jj * 6], -nj.x, -nj.y, -nj.z,
+                                            self ? 0.f : tn.x, self ? 0.f : tn.y, self ? 0.f : tn.z, scale, k2, nk2,
+                                            ki2, acc, sfr, sfi, str_, sti);
         if (self) {   // -1/2 mass matrix of the triangle
             const float m0 = 0.25f * tn.w * p.rw;
 #pragma unroll
