@@ -2249,21 +2249,6 @@ __global__ void k_rc_init(int n, float *x_re, float *x_im, long long stride, RcS
     }
 }
 
-// w = x for the matrices in `want` states (w is solved in place next);
-// active[mat] marks them for the solve
-__global__ void k_rc_copy(int n, const float *x_re, const float *x_im, float *w_re, float *w_im, long long stride,
-                          const RcState *state, int want_lo, int want_hi, int *active) {
-    const int mat = blockIdx.y;
-    const int st = state[mat].st;
-    const bool want = st >= want_lo && st <= want_hi;
-    if (blockIdx.x == 0 && threadIdx.x == 0) active[mat] = want ? 1 : 0;
-    if (!want) return;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        w_re[(size_t)mat * stride + i] = x_re[(size_t)mat * stride + i];
-        w_im[(size_t)mat * stride + i] = x_im[(size_t)mat * stride + i];
-    }
-}
-
 __device__ void block_sum_max(double &sum, float &mx, int &imx) {
     __shared__ double s_sum[32];
     __shared__ float s_mx[32];
@@ -2381,13 +2366,321 @@ __global__ void k_rc_after_h(int n, float *x_re, float *x_im, const float *w_re,
     if (threadIdx.x == 0) state[mat] = sv;
 }
 
-__global__ void k_rc_finish(int batch, const RcState *state, const unsigned *anorm_bits, double *rcond, int *pending) {
+__global__ void k_rc_finish(int batch, const RcState *state, const unsigned *anorm_bits, double *rcond) {
     const int mat = blockIdx.x * blockDim.x + threadIdx.x;
     if (mat >= batch) return;
     const RcState sv = state[mat];
-    if (sv.st != 4) atomicAdd(pending, 1);
     const double an = (double)__uint_as_float(anorm_bits[mat]);
     rcond[mat] = (sv.est != 0.0 && an != 0.0) ? (1.0 / sv.est) / an : 0.0;
+}
+
+// ---------------------------------------------------------------------------
+// Both phases of a solve in one launch, for callers that refine the solution
+// or only estimate with it (k_trsv_wave serves the others, whose roundings
+// stay).  Tickets run through the blocks of the first phase, then of the
+// second, so a block only waits for CTAs that are resident or done; a
+// second-phase block takes its right-hand side from the first phase's
+// mailbox.  While the blocks before it are at work a CTA inverts its 32 x 32
+// diagonal triangle (two 16 x 16 inverses, then their off-diagonal product),
+// so what follows the last block's x is a sum over warps and one 32 x 32
+// product instead of a 32-step sweep with two shuffles a step.  The last two
+// blocks are polled without sleeping.
+//
+// What bounds it: the hand-off of a block through L2 (k_trsv_wave takes 1.3 to
+// 1.8 us a block).  Condition estimate, 13 such solves: n = 162 one matrix 409
+// -> 178 us, n = 1043 1294 -> 615 us, 1043 x 40 1556 -> 1088 us.
+// ---------------------------------------------------------------------------
+struct BothCtl {   // all ones when clear
+    int ticket, abort, pad[2];
+};
+
+__device__ __forceinline__ bool both_wait(const unsigned long long *addr, bool need, unsigned long long &w,
+                                          BothCtl *ctl, int spin_limit, bool near) {
+    w = need ? ld_relaxed_u64(addr) : 0ull;
+    if (__all_sync(0xffffffffu, w != kWaveEmpty)) return true;
+    unsigned ns = 32;
+    for (int spins = 1;; ++spins) {
+        if (!near) {
+            __nanosleep(ns);
+            if (ns < 256) ns <<= 1;
+        }
+        if (w == kWaveEmpty) w = ld_relaxed_u64(addr);
+        if (__all_sync(0xffffffffu, w != kWaveEmpty)) return true;
+        if ((spins & 15) == 0 && __any_sync(0xffffffffu, *(volatile int *)&ctl->abort == 1)) return false;
+        if (spins > spin_limit) {
+            if ((threadIdx.x & 31) == 0) {
+                atomicExch(&ctl->abort, 1);
+                atomicExch(&g_wave_fault, 1);
+            }
+            return false;
+        }
+    }
+}
+
+struct BothShared {
+    float2 t[32][33];      // diagonal triangle as a lower one (an upper phase reversed), 1 on padded rows
+    float2 inv[32][33];
+    float2 w[16][17];
+    float2 dinv[32];
+    __align__(16) float2 v[32];
+    float pr[8][33], pi[8][33];
+    int ticket, abort;
+};
+
+template <bool LOWER, bool UNIT, int TR>
+__device__ __forceinline__ void both_block(BothShared &S, int n, int nblk, int q, const float *Ar, const float *Ai,
+                                           long long lda, const float *br, const float *bi,
+                                           const unsigned long long *rhs, unsigned long long *mb, float *xr, float *xi,
+                                           BothCtl *ctl, int spin_limit) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int b = LOWER ? q : nblk - 1 - q;
+    const int j0 = b * 32, jb = min(32, n - j0);
+    // row r of the block at place r (lower) or 31 - r (upper)
+    for (int e = tid; e < 32 * 32; e += kWaveThreads) {
+        const int r = TR == 0 ? (e >> 5) : (e & 31), c = TR == 0 ? (e & 31) : (e >> 5);
+        float tr = r == c ? 1.f : 0.f, ti = 0.f;
+        if (r < jb && c < jb && (LOWER ? c < r : c > r)) op_at<TR>(Ar, Ai, lda, j0 + r, j0 + c, tr, ti);
+        if (!UNIT && r < jb && c == r) op_at<TR>(Ar, Ai, lda, j0 + r, j0 + r, tr, ti);
+        const int pr = LOWER ? r : 31 - r, pc = LOWER ? c : 31 - c;
+        S.t[pr][pc] = make_float2(tr, ti);
+        S.inv[pr][pc] = make_float2(0.f, 0.f);
+    }
+    __syncthreads();
+    if (warp == 0) {
+        const float2 d = S.t[lane][lane];
+        const float den = 1.0f / fmaf(d.x, d.x, d.y * d.y);
+        S.dinv[lane] = UNIT ? make_float2(1.f, 0.f) : make_float2(d.x * den, -d.y * den);
+    }
+    __syncthreads();
+    if (warp < 2 && lane < 16) {   // column `lane` of the inverse of one 16 x 16 diagonal block
+        const int o = warp * 16;
+        float2 y[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) y[i] = make_float2(i == lane ? 1.f : 0.f, 0.f);
+#pragma unroll
+        for (int k = 0; k < 16; ++k) {
+            if (!UNIT) {
+                const float2 d = S.dinv[o + k];
+                y[k] = make_float2(fmaf(y[k].x, d.x, -y[k].y * d.y), fmaf(y[k].x, d.y, y[k].y * d.x));
+            }
+#pragma unroll
+            for (int i = k + 1; i < 16; ++i) {
+                const float2 l = S.t[o + i][o + k];
+                y[i].x = fmaf(-l.x, y[k].x, fmaf(l.y, y[k].y, y[i].x));
+                y[i].y = fmaf(-l.x, y[k].y, fmaf(-l.y, y[k].x, y[i].y));
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+            if (i >= lane) S.inv[o + i][o + lane] = y[i];
+    }
+    __syncthreads();
+    {
+        const int i = tid >> 4, j = tid & 15;
+        auto product = [&](auto left, auto right) {
+            float2 a = make_float2(0.f, 0.f);
+#pragma unroll 8
+            for (int k = 0; k < 16; ++k) {
+                const float2 l = left(k), r = right(k);
+                a.x = fmaf(l.x, r.x, fmaf(-l.y, r.y, a.x));
+                a.y = fmaf(l.x, r.y, fmaf(l.y, r.x, a.y));
+            }
+            return a;
+        };
+        S.w[i][j] = product([&](int k) { return S.t[16 + i][k]; }, [&](int k) { return S.inv[k][j]; });
+        __syncthreads();
+        const float2 a = product([&](int k) { return S.inv[16 + i][16 + k]; }, [&](int k) { return S.w[k][j]; });
+        S.inv[16 + i][j] = make_float2(-a.x, -a.y);
+    }
+    // op = A: warp w holds rows w + 8k of the block, lanes over the columns of
+    // a finished block; op = A^H: warp w takes factor rows w + 8k of a finished
+    // block, lane i accumulates op-row i of this block
+    const float cs = TR == 2 ? -1.f : 1.f;
+    auto load_a = [&](int qc, float (&pr)[4], float (&pi)[4]) {
+        const int c0 = (LOWER ? qc : nblk - 1 - qc) * 32;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (TR == 0) {
+                const int col = c0 + lane, r = warp + 8 * k;
+                const bool ok = col < n && r < jb;
+                pr[k] = ok ? __ldg(Ar + (size_t)(j0 + r) * lda + col) : 0.f;
+                pi[k] = ok ? __ldg(Ai + (size_t)(j0 + r) * lda + col) : 0.f;
+            } else {
+                const int jr = c0 + warp + 8 * k;
+                const bool ok = jr < n && lane < jb;
+                pr[k] = ok ? __ldg(Ar + (size_t)jr * lda + j0 + lane) : 0.f;
+                pi[k] = ok ? cs * __ldg(Ai + (size_t)jr * lda + j0 + lane) : 0.f;
+            }
+        }
+    };
+    float accr[4] = {0.f, 0.f, 0.f, 0.f}, acci[4] = {0.f, 0.f, 0.f, 0.f};
+    float nr[4], ni[4];   // factor entries of block qc, loaded before its x is waited for
+    bool aborted = false;
+    if (q > 0) load_a(0, nr, ni);
+    for (int qc = 0; qc < q; ++qc) {
+        const int c0 = (LOWER ? qc : nblk - 1 - qc) * 32;
+        const int xi_idx = TR == 0 ? c0 + lane : c0 + warp + 8 * lane;
+        const bool need = TR == 0 ? xi_idx < n : (lane < 4 && xi_idx < n);
+        unsigned long long w;
+        if (!both_wait(mb + (need ? xi_idx : 0), need, w, ctl, spin_limit, q - qc <= 2)) {
+            aborted = true;
+            break;
+        }
+        float pr[4], pi[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) { pr[k] = nr[k]; pi[k] = ni[k]; }
+        if (qc + 1 < q) load_a(qc + 1, nr, ni);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const unsigned long long wk = TR == 0 ? w : __shfl_sync(0xffffffffu, w, k);
+            const float x_r = x_re(wk), x_i = x_im(wk);
+            accr[k] = fmaf(pr[k], x_r, fmaf(-pi[k], x_i, accr[k]));
+            acci[k] = fmaf(pr[k], x_i, fmaf(pi[k], x_r, acci[k]));
+        }
+    }
+    float vr = 0.f, vi = 0.f;
+    if (warp == 0) {
+        if (rhs) {
+            unsigned long long w;
+            if (both_wait(rhs + j0 + min(lane, jb - 1), true, w, ctl, spin_limit, true)) {
+                vr = x_re(w);
+                vi = x_im(w);
+            } else {
+                aborted = true;
+            }
+        } else if (lane < jb) {
+            vr = br[j0 + lane];
+            vi = bi[j0 + lane];
+        }
+    }
+    if (aborted && lane == 0) S.abort = 1;
+    // per-row sums of the finished blocks' contributions
+    if (TR == 0) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const float sr = warp_sum(accr[k]), si = warp_sum(acci[k]);
+            if (lane == 0) { S.pr[0][warp + 8 * k] = sr; S.pi[0][warp + 8 * k] = si; }
+        }
+    } else {
+        S.pr[warp][lane] = (accr[0] + accr[1]) + (accr[2] + accr[3]);
+        S.pi[warp][lane] = (acci[0] + acci[1]) + (acci[2] + acci[3]);
+    }
+    __syncthreads();
+    if (warp != 0) return;
+    float sr = S.pr[0][lane], si = S.pi[0][lane];
+    if (TR != 0) {
+#pragma unroll
+        for (int w = 1; w < 8; ++w) { sr += S.pr[w][lane]; si += S.pi[w][lane]; }
+    }
+    const int place = LOWER ? lane : 31 - lane;
+    S.v[place] = lane < jb ? make_float2(vr - sr, vi - si) : make_float2(0.f, 0.f);
+    __syncwarp();
+    float2 a[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) a[i] = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int k = 0; k < 32; k += 2) {
+        const float4 v = *reinterpret_cast<const float4 *>(&S.v[k]);
+        const float2 l0 = S.inv[place][k], l1 = S.inv[place][k + 1];
+        float2 &a0 = a[k & 2], &a1 = a[(k & 2) + 1];
+        a0.x = fmaf(l0.x, v.x, fmaf(-l0.y, v.y, a0.x));
+        a0.y = fmaf(l0.x, v.y, fmaf(l0.y, v.x, a0.y));
+        a1.x = fmaf(l1.x, v.z, fmaf(-l1.y, v.w, a1.x));
+        a1.y = fmaf(l1.x, v.w, fmaf(l1.y, v.z, a1.y));
+    }
+    vr = (a[0].x + a[1].x) + (a[2].x + a[3].x);
+    vi = (a[0].y + a[1].y) + (a[2].y + a[3].y);
+    if (S.abort == 1) { vr = __int_as_float(0x7fc00000); vi = vr; }
+    if (lane < jb) {
+        st_relaxed_u64(mb + j0 + lane, pack_x(vr, vi));
+        if (xr) {
+            xr[j0 + lane] = vr;
+            xi[j0 + lane] = vi;
+        }
+    }
+}
+
+// System s solves with matrix s % batch; vectors at s * stride.  Skipped: by
+// `active` per system, or where the estimator state of the system is outside
+// [lo, hi].
+template <int TR>
+__global__ void __launch_bounds__(kWaveThreads) k_trsv_both(int n, int nblk, int systems, int batch,
+                                                            const float *__restrict__ lu_re,
+                                                            const float *__restrict__ lu_im, long long lda,
+                                                            long long a_stride, const float *b_re, const float *b_im,
+                                                            long long b_stride, float *x_re_, float *x_im_,
+                                                            long long x_stride, BothCtl *ctl, unsigned long long *mbox,
+                                                            const int *active, const RcState *state, int lo, int hi,
+                                                            int spin_limit) {
+    __shared__ BothShared S;
+    if (threadIdx.x == 0) {
+        S.ticket = atomicAdd(&ctl->ticket, 1) + 1;
+        S.abort = 0;
+    }
+    __syncthreads();
+    const int total = nblk * systems;
+    const int phase = S.ticket >= total, t = S.ticket - phase * total;
+    const int q = t / systems, sys = t - q * systems;
+    if (q >= nblk) return;
+    if (active && active[sys] == 0) return;   // the whole system is skipped; nobody waits on it
+    if (state && (state[sys].st < lo || state[sys].st > hi)) return;
+    const float *Ar = lu_re + (size_t)(sys % batch) * a_stride, *Ai = lu_im + (size_t)(sys % batch) * a_stride;
+    unsigned long long *mb0 = mbox + (size_t)sys * n, *mb1 = mbox + (size_t)(systems + sys) * n;
+    if (phase == 0)
+        both_block<true, TR == 0, TR>(S, n, nblk, q, Ar, Ai, lda, b_re + (size_t)sys * b_stride,
+                                      b_im + (size_t)sys * b_stride, nullptr, mb0, nullptr, nullptr, ctl, spin_limit);
+    else
+        both_block<false, TR != 0, TR>(S, n, nblk, q, Ar, Ai, lda, nullptr, nullptr, mb0, mb1,
+                                       x_re_ + (size_t)sys * x_stride, x_im_ + (size_t)sys * x_stride, ctl, spin_limit);
+}
+
+// The interchanges of piv on a vector, one CTA per system: 32 pivots at a time
+// a lane follows where its top entry, and the entry below that its pivot
+// names, end up (register steps instead of a chain of loads and stores
+// through shared memory per pivot: n = 1043 36 -> 9 us).
+__global__ void __launch_bounds__(kWaveThreads) k_trsv_permute_pos(int n, int batch, const int *piv,
+                                                                   long long piv_stride, float *x_re, float *x_im,
+                                                                   long long stride, const int *active) {
+    extern __shared__ float2 s_vec[];
+    const int sys = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
+    if (active && active[sys] == 0) return;
+    const int *pv = piv + (size_t)(sys % batch) * piv_stride;
+    float *xr = x_re + (size_t)sys * stride, *xi = x_im + (size_t)sys * stride;
+    for (int i = tid; i < n; i += kWaveThreads) s_vec[i] = make_float2(xr[i], xi[i]);
+    __syncthreads();
+    if (tid < 32) {
+        int next = lane < n ? pv[lane] : 0;
+        for (int j0 = 0; j0 < n; j0 += 32) {
+            const int w = min(32, n - j0);
+            int p = next;
+            if (j0 + 32 + lane < n) next = pv[j0 + 32 + lane];
+            if (lane >= w || p < j0 + lane || p >= n) p = j0 + lane;   // no interchange
+            const unsigned same = __match_any_sync(0xffffffffu, p);
+            const bool below = lane < w && p >= j0 + w && (int)__ffs(same) - 1 == lane;
+            int top_pos = j0 + lane, low_pos = below ? p : -1;
+            const float2 top = lane < w ? s_vec[j0 + lane] : make_float2(0.f, 0.f);
+            const float2 low = below ? s_vec[p] : make_float2(0.f, 0.f);
+#pragma unroll 8
+            for (int k = 0; k < 32; ++k) {
+                const int pk = __shfl_sync(0xffffffffu, p, k), j = j0 + k;
+                top_pos = top_pos == j ? pk : (top_pos == pk ? j : top_pos);
+                low_pos = low_pos == j ? pk : (low_pos == pk ? j : low_pos);
+            }
+            __syncwarp();
+            if (lane < w) s_vec[top_pos] = top;
+            if (below) s_vec[low_pos] = low;
+            __syncwarp();
+        }
+    }
+    __syncthreads();
+    for (int i = tid; i < n; i += kWaveThreads) {
+        xr[i] = s_vec[i].x;
+        xi[i] = s_vec[i].y;
+    }
+}
+
+size_t both_scratch_bytes(long long systems, int n) {
+    return sizeof(BothCtl) + 2 * sizeof(unsigned long long) * (size_t)systems * (size_t)n;
 }
 
 // FP64 residual r = b - A x (one warp per row), and per-matrix norms;
@@ -2396,12 +2689,12 @@ __global__ void __launch_bounds__(256) k_residual(int n, const float *a_re, cons
                                                   long long a_stride, const float *b_re, const float *b_im,
                                                   long long b_stride, const float *x_re, const float *x_im,
                                                   long long x_stride, float *r_re, float *r_im, double *norms,
-                                                  const int *active = nullptr) {
+                                                  const int *active = nullptr, int mats = 1 << 30) {
     const int mat = blockIdx.y;
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (warp >= n || (active && !active[mat])) return;
-    const float *Ar = a_re + (size_t)mat * a_stride + (size_t)warp * lda;
-    const float *Ai = a_im + (size_t)mat * a_stride + (size_t)warp * lda;
+    const float *Ar = a_re + (size_t)(mat % mats) * a_stride + (size_t)warp * lda;
+    const float *Ai = a_im + (size_t)(mat % mats) * a_stride + (size_t)warp * lda;
     const float *xr = x_re + (size_t)mat * x_stride, *xi = x_im + (size_t)mat * x_stride;
     double sr = 0, si = 0;
     for (int c = lane; c < n; c += 32) {
@@ -2979,6 +3272,65 @@ int lu_solve(int n, int nrhs, int batch, const float *lu_re, const float *lu_im,
                        nullptr, nullptr, st);
 }
 
+// op(L U) x = b for `systems` vectors (system s with matrix s % batch) by
+// k_trsv_both, for solutions that are refined or only estimated with; piv
+// (optional, TRANS_N only, b == x) applies the interchanges first.
+// `scratch`: both_scratch_bytes(systems, n) that are already all ones, or
+// nullptr to take them from the stream's pool.
+int lu_solve_both(int n, int systems, int batch, const float *lu_re, const float *lu_im, long long lda,
+                  long long a_stride, const int *piv, long long piv_stride, const float *b_re, const float *b_im,
+                  float *x_re, float *x_im, long long stride, int trans, const int *active, const RcState *state,
+                  int lo, int hi, void *scratch, cudaStream_t st) {
+    const int nblk = (n + 31) / 32;
+    if (2LL * nblk * systems >= (1LL << 31)) return fail(HBEM_ERR_ARG, "hbem_lu_solve: too many blocks");
+    if (piv) {
+        const size_t smem = sizeof(float2) * (size_t)n;
+        if (smem > 200 * 1024) return fail(HBEM_ERR_ARG, "hbem_lu_solve: n too large for the staged solve");
+        const int rc = func_opt_in((const void *)k_trsv_permute_pos, 200 * 1024);
+        if (rc != HBEM_OK) return rc;
+        k_trsv_permute_pos<<<systems, kWaveThreads, smem, st>>>(n, batch, piv, piv_stride, x_re, x_im, stride, active);
+        HBEM_LAUNCH_CHECK("k_trsv_permute_pos");
+    }
+    void *mem = scratch;
+    if (!mem) {
+        HBEM_CUDA(cudaMallocAsync(&mem, both_scratch_bytes(systems, n), st));
+        cudaMemsetAsync(mem, 0xff, both_scratch_bytes(systems, n), st);
+    }
+    BothCtl *ctl = static_cast<BothCtl *>(mem);
+    unsigned long long *mbox = reinterpret_cast<unsigned long long *>(ctl + 1);
+    const int spin = tuning(HBEM_TUNE_WAVE_SPIN) > 0 ? tuning(HBEM_TUNE_WAVE_SPIN) : kWaveSpinLimit;
+    const unsigned grid = 2u * (unsigned)nblk * (unsigned)systems;
+    if (trans == HBEM_TRANS_N)
+        k_trsv_both<0><<<grid, kWaveThreads, 0, st>>>(n, nblk, systems, batch, lu_re, lu_im, lda, a_stride, b_re, b_im,
+                                                      stride, x_re, x_im, stride, ctl, mbox, active, state, lo, hi, spin);
+    else
+        k_trsv_both<2><<<grid, kWaveThreads, 0, st>>>(n, nblk, systems, batch, lu_re, lu_im, lda, a_stride, b_re, b_im,
+                                                      stride, x_re, x_im, stride, ctl, mbox, active, state, lo, hi, spin);
+    const cudaError_t e = cudaGetLastError();
+    if (!scratch) cudaFreeAsync(mem, st);
+    if (e != cudaSuccess) return cuda_fail(e, "k_trsv_both");
+    count_launch();
+    return HBEM_OK;
+}
+
+// Solves whose solution is refined: one launch for both phases unless a
+// scheme is forced or the system is small (one CTA solves it).
+bool solve_both_applies(int n) { return tuning(HBEM_TUNE_LU_SOLVE) == 0 && n > kTB && n <= 25600; }
+
+// First solve of a refined solution, `systems` right-hand sides over batch matrices
+int lu_solve_refined(int n, int systems, int batch, const float *lu_re, const float *lu_im, long long lda,
+                     long long a_stride, const int *piv, long long piv_stride, float *x_re, float *x_im,
+                     long long stride, cudaStream_t st) {
+    if (solve_both_applies(n))
+        return lu_solve_both(n, systems, batch, lu_re, lu_im, lda, a_stride, piv, piv_stride, x_re, x_im, x_re, x_im,
+                             stride, HBEM_TRANS_N, nullptr, nullptr, 0, 0, nullptr, st);
+    int rc = HBEM_OK;
+    for (int s0 = 0; s0 < systems && rc == HBEM_OK; s0 += batch)
+        rc = lu_solve(n, 1, batch, lu_re, lu_im, lda, a_stride, piv, piv_stride, x_re + (size_t)s0 * stride,
+                      x_im + (size_t)s0 * stride, 1, stride, HBEM_TRANS_N, st);
+    return rc;
+}
+
 // Reports (and clears) a timed-out wavefront wait; synchronises the stream.
 int wave_fault_check(cudaStream_t st) {
     int h = 0;
@@ -3033,77 +3385,70 @@ int matrix_norm1(int n, int batch, const float *a_re, const float *a_im, long lo
 int lu_rcond(int n, int batch, const float *lu_re, const float *lu_im, long long lda, long long a_stride,
              const float *anorm, double *rcond, cudaStream_t st) {
     constexpr int kItMax = 5;
-    float *x = nullptr, *w = nullptr;
-    RcState *state = nullptr;
-    int *pending = nullptr, *active = nullptr;
-    void *wave = nullptr;
+    // first solve, then kItMax + 1 rounds of an (LU)^H and an (LU) solve: no
+    // host synchronisation, so the estimate can run on its own stream beside
+    // the solves; matrices that finish drop out on the device.  (CLACN2's at
+    // most kItMax (LU)^H solves, then the alternating-sign estimate; one round
+    // to spare.)  The solves' mailboxes are cleared together while they are small.
+    constexpr int kSolves = 1 + 2 * (kItMax + 1);
     const long long stride = n;
-    HBEM_CUDA(cudaMallocAsync((void **)&x, sizeof(float) * 2 * (size_t)batch * n, st));
-    HBEM_CUDA(cudaMallocAsync((void **)&w, sizeof(float) * 2 * (size_t)batch * n, st));
-    HBEM_CUDA(cudaMallocAsync((void **)&state, sizeof(RcState) * batch, st));
-    HBEM_CUDA(cudaMallocAsync((void **)&pending, sizeof(int), st));
-    HBEM_CUDA(cudaMallocAsync((void **)&active, sizeof(int) * batch, st));
-    HBEM_CUDA(cudaMallocAsync(&wave, wave_scratch_bytes(batch, n), st));
-    float *xr = x, *xi = x + (size_t)batch * n, *wr = w, *wi = w + (size_t)batch * n;
+    const size_t vec = (sizeof(float) * 2 * (size_t)batch * n + 255) & ~(size_t)255;
+    const size_t box = (both_scratch_bytes(batch, n) + 255) & ~(size_t)255;
+    const int boxes = box * kSolves <= (32u << 20) ? kSolves : 1;
+    const size_t states = (sizeof(RcState) * batch + 255) & ~(size_t)255;
+    unsigned char *mem = nullptr;
+    HBEM_CUDA(cudaMallocAsync((void **)&mem, 2 * vec + states + box * boxes, st));
+    float *xr = reinterpret_cast<float *>(mem), *xi = xr + (size_t)batch * n;
+    float *wr = reinterpret_cast<float *>(mem + vec), *wi = wr + (size_t)batch * n;
+    RcState *state = reinterpret_cast<RcState *>(mem + 2 * vec);
+    unsigned char *mbox = mem + 2 * vec + states;
     const dim3 gv((n + 255) / 256 < 64 ? (n + 255) / 256 : 64, batch);
-    int rc = HBEM_OK;
+    int rc = HBEM_OK, solves = 0;
     auto launched = [&](const char *what) {
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) { rc = cuda_fail(e, what); return false; }
         count_launch();
         return true;
     };
-    // solves for the matrices k_rc_copy marked active
-    auto solve = [&](int trans) {
-        return lu_solve_ex(n, 1, batch, lu_re, lu_im, lda, a_stride, nullptr, n, wr, wi, 1, stride, trans, active, wave,
-                           st);
+    // op(LU) w = x for the matrices in states lo .. hi
+    auto solve = [&](int trans, int lo, int hi) {
+        unsigned char *b = mbox + (boxes > 1 ? box * solves : 0);
+        if (boxes == 1 || solves == 0) {
+            const cudaError_t e = cudaMemsetAsync(b, 0xff, box * boxes, st);
+            if (e != cudaSuccess) { rc = cuda_fail(e, "rcond mailboxes"); return false; }
+        }
+        ++solves;
+        rc = lu_solve_both(n, batch, batch, lu_re, lu_im, lda, a_stride, nullptr, n, xr, xi, wr, wi, stride, trans,
+                           nullptr, state, lo, hi, b, st);
+        return rc == HBEM_OK;
+    };
+    auto after_a = [&]() {
+        k_rc_after_a<<<batch, 256, 0, st>>>(n, xr, xi, wr, wi, stride, state);
+        return launched("k_rc_after_a");
     };
     k_rc_init<<<gv, 256, 0, st>>>(n, xr, xi, stride, state);
-    // first estimator step: (LU) w = x for every matrix
-    if (launched("k_rc_init")) {
-        k_rc_copy<<<gv, 256, 0, st>>>(n, xr, xi, wr, wi, stride, state, 0, 3, active);
-        if (launched("k_rc_copy")) rc = solve(HBEM_TRANS_N);
-        if (rc == HBEM_OK) { k_rc_after_a<<<batch, 256, 0, st>>>(n, xr, xi, wr, wi, stride, state); launched("k_rc_after_a"); }
-    }
-    // A fixed number of rounds, with no host synchronisation: matrices that
-    // finish drop out on the device (their solves and state updates are
-    // skipped), so the estimate can run on its own stream beside the solves.
-    // Five rounds finish every matrix (CLACN2's at most kItMax (LU)^H solves,
-    // then the alternating-sign estimate); one spare.
-    for (int round = 0; round < kItMax + 1 && rc == HBEM_OK; ++round) {
-        // (LU)^H solves for matrices in state 1, then (LU) solves for states 2 and 3
-        k_rc_copy<<<gv, 256, 0, st>>>(n, xr, xi, wr, wi, stride, state, 1, 1, active);
-        if (!launched("k_rc_copy")) break;
-        rc = solve(HBEM_TRANS_C);
-        if (rc != HBEM_OK) break;
+    bool ok = launched("k_rc_init") && solve(HBEM_TRANS_N, 0, 0) && after_a();
+    for (int round = 0; round < kItMax + 1 && ok; ++round) {
+        ok = solve(HBEM_TRANS_C, 1, 1);
+        if (!ok) break;
         k_rc_after_h<<<batch, 256, 0, st>>>(n, xr, xi, wr, wi, stride, state, kItMax);
-        if (!launched("k_rc_after_h")) break;
-        k_rc_copy<<<gv, 256, 0, st>>>(n, xr, xi, wr, wi, stride, state, 2, 3, active);
-        if (!launched("k_rc_copy")) break;
-        rc = solve(HBEM_TRANS_N);
-        if (rc != HBEM_OK) break;
-        k_rc_after_a<<<batch, 256, 0, st>>>(n, xr, xi, wr, wi, stride, state);
-        if (!launched("k_rc_after_a")) break;
-        // stop once every matrix is done
-        cudaError_t e = cudaMemsetAsync(pending, 0, sizeof(int), st);
-        if (e != cudaSuccess) { rc = cuda_fail(e, "rcond memset"); break; }
-        k_rc_finish<<<(batch + 127) / 128, 128, 0, st>>>(batch, state, reinterpret_cast<const unsigned *>(anorm), rcond,
-                                                         pending);
-        if (!launched("k_rc_finish")) break;
+        ok = launched("k_rc_after_h") && solve(HBEM_TRANS_N, 2, 3) && after_a();
     }
-    cudaFreeAsync(x, st);
-    cudaFreeAsync(w, st);
-    cudaFreeAsync(state, st);
-    cudaFreeAsync(pending, st);
-    cudaFreeAsync(active, st);
-    cudaFreeAsync(wave, st);
+    if (ok) {
+        k_rc_finish<<<(batch + 127) / 128, 128, 0, st>>>(batch, state, reinterpret_cast<const unsigned *>(anorm), rcond);
+        launched("k_rc_finish");
+    }
+    cudaFreeAsync(mem, st);
     return rc;
 }
 
 int refine(int n, int batch, const float *a_re, const float *a_im, long long lda, long long a_stride,
            const float *lu_re, const float *lu_im, long long lu_stride, const int *piv, long long piv_stride,
            const float *b_re, const float *b_im, long long b_stride, float *x_re, float *x_im, long long x_stride,
-           double tol, int max_iter, int *iters, double *resid, cudaStream_t st) {
+           double tol, int max_iter, int *iters, double *resid, cudaStream_t st, int n_src) {
+    // system s (n_src per matrix, source-major) belongs to matrix s % mats
+    const int mats = batch;
+    batch *= n_src;
     // scratch: correction vectors (batch * x_stride * 2 floats) + norms + active flags
     float *d = nullptr;
     double *norms = nullptr;
@@ -3120,7 +3465,7 @@ int refine(int n, int batch, const float *a_re, const float *a_im, long long lda
         if (cudaMemsetAsync(norms, 0, sizeof(double) * 2 * batch, st) != cudaSuccess) { rc = cuda_fail(cudaGetLastError(), "memset"); break; }
         dim3 g((n * 32 + 255) / 256, batch);
         k_residual<<<g, 256, 0, st>>>(n, a_re, a_im, lda, a_stride, b_re, b_im, b_stride, x_re, x_im, x_stride, dr, di, norms,
-                                      it > 0 ? active : nullptr);
+                                      it > 0 ? active : nullptr, mats);
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) { rc = cuda_fail(e, "k_residual"); break; }
         count_launch();
@@ -3142,8 +3487,13 @@ int refine(int n, int batch, const float *a_re, const float *a_im, long long lda
         if (!any) break;
         e = cudaMemcpyAsync(active, h_active.data(), sizeof(int) * batch, cudaMemcpyHostToDevice, st);
         if (e != cudaSuccess) { rc = cuda_fail(e, "refine copy"); break; }
-        rc = lu_solve_ex(n, 1, batch, lu_re, lu_im, lda, lu_stride, piv, piv_stride, dr, di, 1, x_stride, HBEM_TRANS_N,
-                         active, nullptr, st);
+        if (solve_both_applies(n))
+            rc = lu_solve_both(n, batch, mats, lu_re, lu_im, lda, lu_stride, piv, piv_stride, dr, di, dr, di, x_stride,
+                               HBEM_TRANS_N, active, nullptr, 0, 0, nullptr, st);
+        else
+            for (int s0 = 0; s0 < batch && rc == HBEM_OK; s0 += mats)
+                rc = lu_solve_ex(n, 1, mats, lu_re, lu_im, lda, lu_stride, piv, piv_stride, dr + (size_t)s0 * x_stride,
+                                 di + (size_t)s0 * x_stride, 1, x_stride, HBEM_TRANS_N, active + s0, nullptr, st);
         if (rc != HBEM_OK) break;
         k_axpy_active<<<dim3((n + 255) / 256, batch), 256, 0, st>>>(n, x_re, x_im, x_stride, dr, di, active);
         e = cudaGetLastError();
@@ -3196,8 +3546,11 @@ int refine_async(int n, int batch, const float *a_re, const float *a_im, long lo
         if (e != cudaSuccess) { rc = cuda_fail(e, "k_refine_decide"); break; }
         count_launch();
         if (it == max_iter) break;
-        rc = lu_solve_ex(n, 1, batch, lu_re, lu_im, lda, lu_stride, piv, piv_stride, dr, di, 1, x_stride, HBEM_TRANS_N,
-                         active, nullptr, st);
+        rc = solve_both_applies(n)
+                 ? lu_solve_both(n, batch, batch, lu_re, lu_im, lda, lu_stride, piv, piv_stride, dr, di, dr, di, x_stride,
+                                 HBEM_TRANS_N, active, nullptr, 0, 0, nullptr, st)
+                 : lu_solve_ex(n, 1, batch, lu_re, lu_im, lda, lu_stride, piv, piv_stride, dr, di, 1, x_stride,
+                               HBEM_TRANS_N, active, nullptr, st);
         if (rc != HBEM_OK) break;
         k_axpy_active<<<dim3((n + 255) / 256, batch), 256, 0, st>>>(n, x_re, x_im, x_stride, dr, di, active);
         e = cudaGetLastError();
@@ -3367,7 +3720,7 @@ extern "C" int hbem_refine(int n, int batch, const float *a_re, const float *a_i
     if (lda < n || a_stride < lda * (long long)n || lu_stride < lda * (long long)n || piv_stride < n)
         return fail(HBEM_ERR_ARG, "hbem_refine: lda/a_stride/lu_stride/piv_stride too small");
     return refine(n, batch, a_re, a_im, lda, a_stride, lu_re, lu_im, lu_stride, piv, piv_stride, b_re, b_im, b_stride,
-                  x_re, x_im, x_stride, tol, max_iter, iters, resid, reinterpret_cast<cudaStream_t>(stream));
+                  x_re, x_im, x_stride, tol, max_iter, iters, resid, reinterpret_cast<cudaStream_t>(stream), 1);
 }
 
 extern "C" int hbem_refine_async(int n, int batch, const float *a_re, const float *a_im, long long lda,

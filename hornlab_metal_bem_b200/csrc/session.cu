@@ -350,35 +350,41 @@ void cluster_order(const std::vector<int> &l2g, int n_dof, const std::vector<int
     std::vector<char> used(T, 0);
     // stamps: the chunk, tile and previous tile a dof belongs to last
     std::vector<int> chunk_of(n_dof, -1), tile_of(n_dof, -1);
-    std::vector<int> chunk, tile, prev_tile;
+    // last_of: the position of the last triangle with that dof; seen: the last
+    // position a triangle was a candidate for
+    std::vector<int> chunk, tile, prev_tile, last_of(n_dof, -2), seen(T, -1);
     order.clear();
     order.reserve(T);
-    int next_seed = 0, last = -1;
+    int next_seed = 0;
     while ((int)order.size() < T) {
         const int pos = (int)order.size(), ci = pos / kChunk, ti = pos / kTestTile;
         if (pos % kTestTile == 0) { prev_tile.swap(tile); tile.clear(); }
         if (pos % kChunk == 0) chunk.clear();
-        int best = -1, key[4] = {0, 0, 0, 0};
+        int best = -1;
+        long long best_key = 0;
         const std::vector<int> *pools[3] = {&chunk, &tile, &prev_tile};
         for (int lvl = 0; lvl < 3 && best < 0; ++lvl)
             for (int v : *pools[lvl])
                 for (int e = start[v]; e < start[v + 1]; ++e) {
                     const int u = inc[e];
-                    if (used[u]) continue;
+                    if (used[u] || seen[u] == pos) continue;
+                    seen[u] = pos;
                     int new_c = 0, new_t = 0, with_last = 0, left = 0;
                     for (int l = 0; l < 3; ++l) {
                         const int d = l2g[3 * u + l];
                         new_c += chunk_of[d] != ci;
                         new_t += tile_of[d] != ti;
+                        with_last += last_of[d] == pos - 1;
                         left += open[d];
-                        for (int m = 0; m < 3 && last >= 0; ++m) with_last += l2g[3 * last + m] == d;
                     }
-                    int k[4] = {0, 0, left, rank[u]};
-                    if (lvl == 0) { k[0] = new_c * 8 + new_t; k[1] = -with_last; }
-                    else if (lvl == 1) { k[0] = new_t; k[1] = left; k[2] = -with_last; }
-                    if (best < 0 || std::lexicographical_compare(k, k + 4, key, key + 4)) {
+                    // lexicographic: smallest first
+                    const int k0 = lvl == 0 ? new_c * 4 + new_t : (lvl == 1 ? new_t : 0);
+                    const int k1 = lvl == 0 ? 3 - with_last : left, k2 = lvl == 0 ? left : 3 - with_last;
+                    const long long key = (((long long)k0 << 10 | std::min(k1, 1023)) << 10 | std::min(k2, 1023)) << 32 |
+                                          (unsigned)rank[u];
+                    if (best < 0 || key < best_key) {
                         best = u;
-                        std::copy(k, k + 4, key);
+                        best_key = key;
                     }
                 }
         if (best < 0) {
@@ -387,10 +393,10 @@ void cluster_order(const std::vector<int> &l2g, int n_dof, const std::vector<int
         }
         used[best] = 1;
         order.push_back(best);
-        last = best;
         for (int l = 0; l < 3; ++l) {
             const int d = l2g[3 * best + l];
             --open[d];
+            last_of[d] = pos;
             if (chunk_of[d] != ci) { chunk_of[d] = ci; chunk.push_back(d); }
             if (tile_of[d] != ti) { tile_of[d] = ti; tile.push_back(d); }
         }

@@ -28,7 +28,10 @@ int lu_rcond(int n, int batch, const float *lu_re, const float *lu_im, long long
 int refine(int n, int batch, const float *a_re, const float *a_im, long long lda, long long a_stride,
            const float *lu_re, const float *lu_im, long long lu_stride, const int *piv, long long piv_stride,
            const float *b_re, const float *b_im, long long b_stride, float *x_re, float *x_im, long long x_stride,
-           double tol, int max_iter, int *iters, double *resid, cudaStream_t st);
+           double tol, int max_iter, int *iters, double *resid, cudaStream_t st, int n_src = 1);
+int lu_solve_refined(int n, int systems, int batch, const float *lu_re, const float *lu_im, long long lda,
+                     long long a_stride, const int *piv, long long piv_stride, float *x_re, float *x_im,
+                     long long stride, cudaStream_t st);
 int wave_fault_check(cudaStream_t st);
 int launch_field(Session &s, int n_freq, const float *k_re, const float *p_re, const float *p_im, long long p_stride,
                  const float *q_re, const float *q_im, long long q_stride, const float *obs, int n_obs, float *out_re,
@@ -268,16 +271,16 @@ static int solve_batch_impl(hbem_session *h, int n_freq, int n_src, const float 
                 if (rc == HBEM_OK) ok(cudaEventRecord(s->aux_join, s->aux), "join");
                 if (rc != HBEM_OK) break;
             }
-            for (int sv = 0; sv < n_src && rc == HBEM_OK; ++sv)
+            if (do_refine)
+                rc = lu_solve_refined((int)n, n_src * nf, nf, ar, ai, lda, na, dpiv, (long long)n, xr, xi, (long long)n, st);
+            for (int sv = 0; sv < n_src && rc == HBEM_OK && !do_refine; ++sv)
                 rc = lu_solve((int)n, 1, nf, ar, ai, lda, na, dpiv, (long long)n, xr + sv * xs, xi + sv * xs,
                               1, (long long)n, HBEM_TRANS_N, st);
             if (rc != HBEM_OK) break;
         }
         if (do_refine) {
-            for (int sv = 0; sv < n_src && rc == HBEM_OK; ++sv)
-                rc = refine((int)n, nf, a0r, a0i, lda, na, ar, ai, na, dpiv, (long long)n, br + sv * xs,
-                            bi + sv * xs, (long long)n, xr + sv * xs, xi + sv * xs, (long long)n, tol, max_iter,
-                            diters + (size_t)sv * nf, dres + (size_t)sv * nf, st);
+            rc = refine((int)n, nf, a0r, a0i, lda, na, ar, ai, na, dpiv, (long long)n, br, bi, (long long)n, xr, xi,
+                        (long long)n, tol, max_iter, diters, dres, st, n_src);
             if (rc != HBEM_OK) break;
         }
         ok(cudaEventRecord(ev[2], st), "cudaEventRecord");

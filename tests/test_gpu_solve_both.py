@@ -1,0 +1,60 @@
+"""Solves by one launch for both triangular phases (refinement and condition estimate) at the edges of its 32-row
+blocks, against LAPACK.
+
+Refined solutions: hbem_refine stops at a relative residual of 1e-7 and keeps x in FP32 (2^-24 of each entry); the
+matrices' condition numbers stay below 30 (diagonally dominant), so 30 * 1e-7 + 6e-8 < 4e-6.  Condition estimates:
+cgecon's own on the same matrix, 1 % apart as the estimator's vectors are rounded differently."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+if not torch.cuda.is_available():  # pragma: no cover - CPU containers
+    pytest.skip("needs a CUDA device", allow_module_level=True)
+
+from scipy.linalg import lapack  # noqa: E402
+
+from hornlab_metal_bem_b200.native import HBEM_PREC_TF32X3, _stream_ptr, _t_ptr, check, load_library  # noqa: E402
+
+
+def _parts(z):
+    return (torch.tensor(np.ascontiguousarray(z.real), dtype=torch.float32).cuda(),
+            torch.tensor(np.ascontiguousarray(z.imag), dtype=torch.float32).cuda())
+
+
+@pytest.mark.parametrize("n,batch", [(1, 2), (2, 1), (31, 3), (32, 1), (33, 2), (64, 1), (129, 5), (160, 1), (161, 2),
+                                     (513, 3)])
+def test_refined_solution_and_condition_estimate(n, batch):
+    lib = load_library()
+    rng = np.random.default_rng(n)
+    A = (rng.standard_normal((batch, n, n)) + 1j * rng.standard_normal((batch, n, n))).astype(np.complex64)
+    A += (4.0 * np.sqrt(n)) * np.eye(n, dtype=np.complex64)[rng.permutation(n)]   # interchanges off the diagonal
+    b = (rng.standard_normal((batch, n)) + 1j * rng.standard_normal((batch, n))).astype(np.complex64)
+    A0r, A0i = _parts(A)
+    Ar, Ai = A0r.clone(), A0i.clone()
+    br, bi = _parts(b)
+    xr, xi = torch.zeros_like(br), torch.zeros_like(bi)
+    piv = torch.empty((batch, n), dtype=torch.int32, device="cuda")
+    info = torch.empty(batch, dtype=torch.int32, device="cuda")
+    anorm = torch.empty(batch, dtype=torch.float32, device="cuda")
+    rcond = torch.empty(batch, dtype=torch.float64, device="cuda")
+    st = _stream_ptr()
+    check(lib.hbem_matrix_norm1(n, batch, _t_ptr(Ar), _t_ptr(Ai), n, n * n, _t_ptr(anorm), st), "hbem_matrix_norm1")
+    check(lib.hbem_lu_factor(n, batch, _t_ptr(Ar), _t_ptr(Ai), n, n * n, _t_ptr(piv), n, _t_ptr(info), HBEM_PREC_TF32X3,
+                             st), "hbem_lu_factor")
+    check(lib.hbem_lu_rcond(n, batch, _t_ptr(Ar), _t_ptr(Ai), n, n * n, _t_ptr(anorm), _t_ptr(rcond), st),
+          "hbem_lu_rcond")
+    # from x = 0 the first pass solves for b itself
+    check(lib.hbem_refine(n, batch, _t_ptr(A0r), _t_ptr(A0i), n, n * n, _t_ptr(Ar), _t_ptr(Ai), n * n, _t_ptr(piv), n,
+                          _t_ptr(br), _t_ptr(bi), n, _t_ptr(xr), _t_ptr(xi), n, 1e-7, 6, None, None, st), "hbem_refine")
+    assert not info.cpu().numpy().any()
+    x = xr.double().cpu().numpy() + 1j * xi.double().cpu().numpy()
+    for m in range(batch):
+        ref = np.linalg.solve(A[m].astype(np.complex128), b[m].astype(np.complex128))
+        assert np.linalg.norm(x[m] - ref) <= 4e-6 * np.linalg.norm(ref)
+        lu, _, _ = lapack.cgetrf(A[m])
+        want, _ = lapack.cgecon(lu, np.abs(A[m]).sum(0).max().astype(np.float32), norm="1")
+        assert abs(float(rcond[m]) - want) <= 1e-2 * want
