@@ -42,7 +42,8 @@ namespace {
 constexpr int kBwdTest = 32;
 constexpr int kBwdTrial = 64;
 constexpr int kBwdThreads = 256;
-constexpr int kBwdMaxF = 16;        // frequencies staged per launch
+constexpr int kBwdMaxF = 20;        // frequencies staged per launch (two CTAs an SM)
+constexpr int kBwdTouchF = 16;      // frequencies per launch of the touching pairs
 constexpr float kTwoPi = 6.28318530717958647692f;
 
 __device__ __forceinline__ float bqx(int q) {
@@ -58,9 +59,22 @@ __device__ __forceinline__ float rnd(float t) {
     return __fsub_rn(__fadd_rn(t, big), big);
 }
 
+__device__ __forceinline__ float rsqrt_ftz(float x) {
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+// barycentrics and weight of the six rule points
+__constant__ float4 c_rule[6] = {
+    {1.0f - HBEM_QX0 - HBEM_QY0, HBEM_QX0, HBEM_QY0, HBEM_QWA}, {1.0f - HBEM_QX1 - HBEM_QY1, HBEM_QX1, HBEM_QY1, HBEM_QWB},
+    {1.0f - HBEM_QX2 - HBEM_QY2, HBEM_QX2, HBEM_QY2, HBEM_QWA}, {1.0f - HBEM_QX3 - HBEM_QY3, HBEM_QX3, HBEM_QY3, HBEM_QWA},
+    {1.0f - HBEM_QX4 - HBEM_QY4, HBEM_QX4, HBEM_QY4, HBEM_QWB}, {1.0f - HBEM_QX5 - HBEM_QY5, HBEM_QX5, HBEM_QY5, HBEM_QWB}};
+
 struct Freqs {
-    float k[kBwdMaxF];
-    float kt[kBwdMaxF];   // k / (2 pi)
+    alignas(8) float k[kBwdMaxF];
+    alignas(8) float kk[kBwdMaxF];   // k^2
+    alignas(8) float kt[kBwdMaxF];   // k / (2 pi)
 };
 
 // Running sums of one (test, trial) pair or one sample set.
@@ -80,6 +94,19 @@ __device__ __forceinline__ void acc_zero(PairAcc &a) {
     a.gn[0] = a.gn[1] = a.gn[2] = 0.f;
     a.gjs = a.gjt = 0.f;
 }
+
+// Regular pairs: a geometric sample needs five sums over the frequencies, none
+// of which carries its geometry: with u_p = -conj(lambda) p, u_q = conj(lambda) q and
+// W = -u_p e^{ikr}, Q = u_q e^{ikr} (one rotation each)
+//   S1 = sum Re W, S2 = sum k Im W, S3 = sum k^2 Re W,
+//   T1 = sum Re Q, T2 = sum k Im Q,
+// and s = e^{ikr} (-1 + ikr) / r^3, s' = e^{ikr} (3/r - k^2 r - 3ik) / r^3,
+// G = e^{ikr} / r give
+//   sum Re u_p s  = (S1 + r S2) / r^3,   sum Re u_p s' = -(3 S1 / r + 3 S2 - r S3) / r^3,
+//   sum Re u_q s  = -(T1 + r T2) / r^3,  sum Re u_q G  = T1 / r.
+struct FreqSums {
+    float s1, s2, s3, t1, t2;
+};
 
 // One geometric sample: d = y - x, trial area normal N (|N| = js), test
 // barycentrics tb, trial barycentrics sb, weight w (includes J_tau's
@@ -203,15 +230,25 @@ struct BwdArgs {
 
 // ---------------------------------------------------------------------------
 // Regular pairs: 32 test x 64 trial triangles per CTA, thread (lane, warp)
-// takes test lane and trial warp + 8 j, all staged frequencies per sample.
-// Touching pairs are skipped (their Duffy rule replaces the regular rule).
+// takes test lane and trial warp + 8 j, all staged frequencies per sample, two
+// at a time as packed FP32 pairs (lambda and p are staged as (re, re, im, im)
+// of a pair of frequencies).  Touching pairs are skipped (their Duffy rule
+// replaces the regular rule); the Neumann terms only run where the trial
+// triangle is driven.
+// The trial triangle's gradient is a warp total and the test triangle's stays in
+// registers (per-pair shared atomics, 32 lanes on one address, were a third of
+// the instructions).  Bound: issue, 14 slots of the FP32 pipe per sample and
+// frequency beside the MUFU pipe's sine and cosine.  4160 triangles x 20
+// frequencies: 40.8 -> 16 ms with the touching pairs.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(kBwdThreads) k_asm_bwd(const __grid_constant__ BwdArgs a) {
+__global__ void __launch_bounds__(kBwdThreads, 2) k_asm_bwd(const __grid_constant__ BwdArgs a) {
     extern __shared__ float sh[];
     const int nf = a.nf;
-    float *sL = sh;                                        // [f][q][test][2]
-    float *sP = sL + (size_t)nf * 6 * kBwdTest * 2;        // [f][q][trial][2]
-    float *sQ = sP + (size_t)nf * 6 * kBwdTrial * 2;       // [f][trial][2]
+    const int np = (nf + 1) / 2;                           // frequency pairs (an odd last one with zero lambda)
+    float *sL = sh;                                        // [pair][q][test] (re, re, im, im)
+    float *sP = sL + (size_t)np * 6 * kBwdTest * 4;        // [pair][q][trial]
+    float *sQ = sP + (size_t)np * 6 * kBwdTrial * 4;       // [pair][trial]
+    __shared__ int sDriven[kBwdTrial];
     __shared__ float sTV[kBwdTest][9], sSV[kBwdTrial][9];
     __shared__ float gT[kBwdTest][9], gS[kBwdTrial][9];
     const int T = a.T, V = a.V;
@@ -229,11 +266,11 @@ __global__ void __launch_bounds__(kBwdThreads) k_asm_bwd(const __grid_constant__
         sSV[i][lc] = t < T ? a.verts[(size_t)c * V + a.tris[(size_t)l * T + t]] : 0.f;
         gS[i][lc] = 0.f;
     }
-    for (int e = tid; e < nf * 6 * kBwdTest; e += kBwdThreads) {
+    for (int e = tid; e < 2 * np * 6 * kBwdTest; e += kBwdThreads) {
         const int f = e / (6 * kBwdTest), rem = e - f * 6 * kBwdTest, q = rem / kBwdTest, i = rem - q * kBwdTest;
         const int t = t0 + i;
         float lr = 0.f, li = 0.f;
-        if (t < T) {
+        if (t < T && f < nf) {
             const float b[3] = {1.f - bqx(q) - bqy(q), bqx(q), bqy(q)};
 #pragma unroll
             for (int l = 0; l < 3; ++l) {
@@ -242,14 +279,15 @@ __global__ void __launch_bounds__(kBwdThreads) k_asm_bwd(const __grid_constant__
                 li = fmaf(-b[l], a.lam_im[(size_t)f * a.lam_stride + d], li);   // conj(lambda)
             }
         }
-        sL[2 * e] = lr;
-        sL[2 * e + 1] = li;
+        float *to = sL + 4 * (((f >> 1) * 6 + q) * kBwdTest + i) + (f & 1);
+        to[0] = lr;
+        to[2] = li;
     }
-    for (int e = tid; e < nf * 6 * kBwdTrial; e += kBwdThreads) {
+    for (int e = tid; e < 2 * np * 6 * kBwdTrial; e += kBwdThreads) {
         const int f = e / (6 * kBwdTrial), rem = e - f * 6 * kBwdTrial, q = rem / kBwdTrial, i = rem - q * kBwdTrial;
         const int t = s0 + i;
         float pr = 0.f, pi = 0.f;
-        if (t < T) {
+        if (t < T && f < nf) {
             const float b[3] = {1.f - bqx(q) - bqy(q), bqx(q), bqy(q)};
 #pragma unroll
             for (int l = 0; l < 3; ++l) {
@@ -258,77 +296,164 @@ __global__ void __launch_bounds__(kBwdThreads) k_asm_bwd(const __grid_constant__
                 pi = fmaf(b[l], a.p_im[(size_t)f * a.p_stride + d], pi);
             }
         }
-        sP[2 * e] = pr;
-        sP[2 * e + 1] = pi;
+        float *to = sP + 4 * (((f >> 1) * 6 + q) * kBwdTrial + i) + (f & 1);
+        to[0] = pr;
+        to[2] = pi;
     }
-    for (int e = tid; e < nf * kBwdTrial; e += kBwdThreads) {
-        const int f = e / kBwdTrial, i = e - f * kBwdTrial;
+    for (int i = tid; i < kBwdTrial; i += kBwdThreads) {
         const int t = s0 + i;
-        sQ[2 * e] = t < T && a.q_re ? a.q_re[(size_t)f * a.q_stride + t] : 0.f;
-        sQ[2 * e + 1] = t < T && a.q_im ? a.q_im[(size_t)f * a.q_stride + t] : 0.f;
+        int driven = 0;
+        for (int f = 0; f < 2 * np; ++f) {
+            const bool in = t < T && f < nf && a.q_re && a.q_im;
+            const float qr = in ? a.q_re[(size_t)f * a.q_stride + t] : 0.f;
+            const float qi = in ? a.q_im[(size_t)f * a.q_stride + t] : 0.f;
+            float *to = sQ + 4 * ((f >> 1) * kBwdTrial + i) + (f & 1);
+            to[0] = qr;
+            to[2] = qi;
+            driven |= qr != 0.f || qi != 0.f;
+        }
+        sDriven[i] = driven;
     }
     __syncthreads();
     const int ti = lane;
     const int tt = t0 + ti;
-    if (tt < T) {
-        float TV[3][3];
+    float TV[3][3];
+#pragma unroll
+    for (int l = 0; l < 3; ++l)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) TV[l][c] = sTV[ti][3 * l + c];
+    float Nt[3], jt;
+    area_normal(TV, Nt, jt);
+    float gt_sum[3][3];   // this lane's test triangle, over the warp's trial triangles
+#pragma unroll
+    for (int l = 0; l < 3; ++l)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) gt_sum[l][c] = 0.f;
+    for (int si = warp; si < kBwdTrial; si += kBwdThreads / 32) {
+        const int st = s0 + si;
+        if (st >= T) break;
+        // every lane goes through the pair (the trial sums are warp totals);
+        // lanes past the mesh and touching pairs contribute zero
+        const size_t bit = (size_t)min(tt, T - 1) * T + st;
+        const bool counts = tt < T && !((a.sing[bit >> 5] >> (bit & 31)) & 1u);
+        if (!__any_sync(0xffffffffu, counts)) continue;
+        float SV[3][3];
 #pragma unroll
         for (int l = 0; l < 3; ++l)
 #pragma unroll
-            for (int c = 0; c < 3; ++c) TV[l][c] = sTV[ti][3 * l + c];
-        float Nt[3], jt;
-        area_normal(TV, Nt, jt);
-        for (int si = warp; si < kBwdTrial; si += kBwdThreads / 32) {
-            const int st = s0 + si;
-            if (st >= T) break;
-            const size_t bit = (size_t)tt * T + st;
-            if ((a.sing[bit >> 5] >> (bit & 31)) & 1u) continue;
-            float SV[3][3];
-#pragma unroll
-            for (int l = 0; l < 3; ++l)
-#pragma unroll
-                for (int c = 0; c < 3; ++c) SV[l][c] = sSV[si][3 * l + c];
-            float N[3], js;
-            area_normal(SV, N, js);
-            PairAcc acc;
-            acc_zero(acc);
-            for (int qa = 0; qa < 6; ++qa) {
-                const float tb[3] = {1.f - bqx(qa) - bqy(qa), bqx(qa), bqy(qa)};
-                float x[3];
-#pragma unroll
-                for (int c = 0; c < 3; ++c) x[c] = tb[0] * TV[0][c] + tb[1] * TV[1][c] + tb[2] * TV[2][c];
-                const float wa = bqw(qa);
+            for (int c = 0; c < 3; ++c) SV[l][c] = sSV[si][3 * l + c];
+        float N[3], js;
+        area_normal(SV, N, js);
+        const bool driven = sDriven[si] != 0;
+        PairAcc acc;
+        acc_zero(acc);
 #pragma unroll 1
-                for (int qb = 0; qb < 6; ++qb) {
-                    const float sb[3] = {1.f - bqx(qb) - bqy(qb), bqx(qb), bqy(qb)};
-                    float y[3];
+        for (int qa = 0; qa < 6; ++qa) {
+            const float4 ra = c_rule[qa];   // barycentrics and weight
+            const float tb[3] = {ra.x, ra.y, ra.z};
+            float x[3], gx[3] = {0.f, 0.f, 0.f};
 #pragma unroll
-                    for (int c = 0; c < 3; ++c) y[c] = sb[0] * SV[0][c] + sb[1] * SV[1][c] + sb[2] * SV[2][c];
-                    auto uw = [&](int f, float &upr, float &upi, float &uqr, float &uqi) {
-                        const float lr = sL[2 * ((f * 6 + qa) * kBwdTest + ti)];
-                        const float li = sL[2 * ((f * 6 + qa) * kBwdTest + ti) + 1];
-                        const float pr = sP[2 * ((f * 6 + qb) * kBwdTrial + si)];
-                        const float pi = sP[2 * ((f * 6 + qb) * kBwdTrial + si) + 1];
-                        const float qr = sQ[2 * (f * kBwdTrial + si)], qi = sQ[2 * (f * kBwdTrial + si) + 1];
-                        upr = -(lr * pr - li * pi);
-                        upi = -(lr * pi + li * pr);
-                        uqr = lr * qr - li * qi;
-                        uqi = lr * qi + li * qr;
-                    };
-                    bwd_sample(acc, y[0] - x[0], y[1] - x[1], y[2] - x[2], N, js, tb, sb, wa * bqw(qb), jt, a.fq, nf, uw);
+            for (int c = 0; c < 3; ++c) x[c] = tb[0] * TV[0][c] + tb[1] * TV[1][c] + tb[2] * TV[2][c];
+            const float4 *L = reinterpret_cast<const float4 *>(sL) + qa * kBwdTest + ti;
+#pragma unroll 1
+            for (int qb = 0; qb < 6; ++qb) {
+                const float4 rb = c_rule[qb];
+                const float sb[3] = {rb.x, rb.y, rb.z};
+                float y[3];
+#pragma unroll
+                for (int c = 0; c < 3; ++c) y[c] = sb[0] * SV[0][c] + sb[1] * SV[1][c] + sb[2] * SV[2][c];
+                const float dx = y[0] - x[0], dy = y[1] - x[1], dz = y[2] - x[2];
+                const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+                float u1 = rsqrt_ftz(r2);
+                u1 = r2 > 1.0e-14f ? u1 : 0.f;   // such a sample adds nothing (every term has a factor u1 or d)
+                const float r = r2 * u1;
+                const float4 *P = reinterpret_cast<const float4 *>(sP) + qb * kBwdTrial + si;
+                float2 s1 = make_float2(0.f, 0.f), s2 = s1, s3 = s1, t1 = s1, t2 = s1;
+                const float2 rr = make_float2(r, r);
+                auto freq_pair = [&](int fp, bool with_q) {
+                    const float2 k = *reinterpret_cast<const float2 *>(&a.fq.k[2 * fp]);
+                    const float2 kk = *reinterpret_cast<const float2 *>(&a.fq.kk[2 * fp]);
+                    const float4 l = L[fp * 6 * kBwdTest], p = P[fp * 6 * kBwdTrial];
+                    const float2 lr = make_float2(l.x, l.y), li = make_float2(l.z, l.w), nli = make_float2(-l.z, -l.w);
+                    const float2 pr = make_float2(p.x, p.y), pi = make_float2(p.z, p.w);
+                    // phase in turns, reduced to [-1/2, 1/2]: one rounding of r k / 2 pi
+                    float2 t = __fmul2_rn(rr, *reinterpret_cast<const float2 *>(&a.fq.kt[2 * fp]));
+                    t = make_float2(t.x - rnd(t.x), t.y - rnd(t.y));
+                    float2 sn, cs;
+                    __sincosf(t.x * kTwoPi, &sn.x, &cs.x);
+                    __sincosf(t.y * kTwoPi, &sn.y, &cs.y);
+                    const float2 nsn = make_float2(-sn.x, -sn.y);
+                    // conj(lambda) p, then its rotation by e^{ikr}
+                    const float2 mr = __ffma2_rn(lr, pr, __fmul2_rn(nli, pi));
+                    const float2 mi = __ffma2_rn(lr, pi, __fmul2_rn(li, pr));
+                    const float2 w1 = __ffma2_rn(mr, cs, __fmul2_rn(mi, nsn));
+                    const float2 w2 = __ffma2_rn(mr, sn, __fmul2_rn(mi, cs));
+                    s1 = __fadd2_rn(s1, w1);
+                    s2 = __ffma2_rn(k, w2, s2);
+                    s3 = __ffma2_rn(kk, w1, s3);
+                    if (with_q) {
+                        const float4 qv = reinterpret_cast<const float4 *>(sQ)[fp * kBwdTrial + si];
+                        const float2 qr = make_float2(qv.x, qv.y), qi = make_float2(qv.z, qv.w);
+                        const float2 nr = __ffma2_rn(lr, qr, __fmul2_rn(nli, qi));
+                        const float2 ni = __ffma2_rn(lr, qi, __fmul2_rn(li, qr));
+                        t1 = __fadd2_rn(t1, __ffma2_rn(nr, cs, __fmul2_rn(ni, nsn)));
+                        t2 = __ffma2_rn(k, __ffma2_rn(nr, sn, __fmul2_rn(ni, cs)), t2);
+                    }
+                };
+                if (driven) {
+#pragma unroll 1
+                    for (int fp = 0; fp < np; ++fp) freq_pair(fp, true);
+                } else {
+#pragma unroll 2
+                    for (int fp = 0; fp < np; ++fp) freq_pair(fp, false);
                 }
-            }
-            float gt[3][3], gs[3][3];
-            finish_pair(acc, TV, SV, N, js, gt, gs, true);
-#pragma unroll
-            for (int l = 0; l < 3; ++l)
+                const float S1 = s1.x + s1.y, S2 = s2.x + s2.y, S3 = s3.x + s3.y, T1 = t1.x + t1.y, T2 = t2.x + t2.y;
+                const float u3 = u1 * u1 * u1;
+                const float dn = fmaf(dx, N[0], fmaf(dy, N[1], dz * N[2]));
+                const float An = u3 * fmaf(r, S2, S1);
+                const float ps = -u3 * fmaf(3.f, fmaf(u1, S1, S2), -r * S3);
+                const float qs = -u3 * fmaf(r, T2, T1);
+                const float Aj = u1 * T1;
+                const float Ad = fmaf(ps, dn * u1, js * qs);
+                const float Af = fmaf(An, dn, js * Aj);
+                const float w = ra.w * rb.w, W = w * jt;
+                const float gd[3] = {W * fmaf(Ad, dx, An * N[0]), W * fmaf(Ad, dy, An * N[1]),
+                                     W * fmaf(Ad, dz, An * N[2])};
 #pragma unroll
                 for (int c = 0; c < 3; ++c) {
-                    atomicAdd(&gT[ti][3 * l + c], gt[l][c]);
-                    atomicAdd(&gS[si][3 * l + c], gs[l][c]);
+                    gx[c] += gd[c];
+#pragma unroll
+                    for (int l = 0; l < 3; ++l) acc.gy[l][c] = fmaf(sb[l], gd[c], acc.gy[l][c]);
                 }
+                const float wn = W * An;
+                acc.gn[0] = fmaf(wn, dx, acc.gn[0]);
+                acc.gn[1] = fmaf(wn, dy, acc.gn[1]);
+                acc.gn[2] = fmaf(wn, dz, acc.gn[2]);
+                acc.gjs = fmaf(W, Aj, acc.gjs);
+                acc.gjt = fmaf(w, Af, acc.gjt);
+            }
+#pragma unroll
+            for (int l = 0; l < 3; ++l)
+#pragma unroll
+                for (int c = 0; c < 3; ++c) acc.gx[l][c] = fmaf(-tb[l], gx[c], acc.gx[l][c]);
         }
+        float gt[3][3], gs[3][3];
+        finish_pair(acc, TV, SV, N, js, gt, gs, true);
+#pragma unroll
+        for (int l = 0; l < 3; ++l)
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                gt_sum[l][c] += counts ? gt[l][c] : 0.f;
+                float v = counts ? gs[l][c] : 0.f;
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+                if (lane == 0) gS[si][3 * l + c] = v;   // one warp per trial triangle
+            }
     }
+#pragma unroll
+    for (int l = 0; l < 3; ++l)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) atomicAdd(&gT[ti][3 * l + c], gt_sum[l][c]);
     __syncthreads();
     for (int e = tid; e < kBwdTest * 9; e += kBwdThreads) {
         const int i = e / 9, lc = e - 9 * i, l = lc / 3, c = lc - 3 * l;
@@ -635,6 +760,7 @@ __global__ void k_field_bwd(const __grid_constant__ FieldBwdArgs a) {
 void fill_freqs(Freqs &fq, const float *k_re, int f0, int nf) {
     for (int f = 0; f < nf; ++f) {
         fq.k[f] = k_re[f0 + f];
+        fq.kk[f] = k_re[f0 + f] * k_re[f0 + f];
         fq.kt[f] = (float)((double)k_re[f0 + f] / (2.0 * 3.14159265358979323846));
     }
 }
@@ -789,8 +915,9 @@ extern "C" int hbem_assemble_backward(hbem_session *h, int n_freq, const float *
         const int rc = func_opt_in((const void *)k_asm_bwd, 200 * 1024);
         if (rc != HBEM_OK) return rc;
     }
-    for (int f0 = 0; f0 < n_freq; f0 += kBwdMaxF) {
-        const int nf = std::min(kBwdMaxF, n_freq - f0);
+    // regular pairs kBwdMaxF frequencies a launch; touching pairs 16, whose FP32
+    // lane sums cancel (another grouping of them moves the gradient by 6e-6)
+    auto args = [&](int f0, int nf) {
         BwdArgs a{};
         a.verts = s->d_verts; a.tris = s->d_tris; a.l2g = s->d_l2g;
         a.lam_re = lam_re + (size_t)f0 * lam_stride; a.lam_im = lam_im + (size_t)f0 * lam_stride;
@@ -799,10 +926,18 @@ extern "C" int hbem_assemble_backward(hbem_session *h, int n_freq, const float *
         a.lam_stride = lam_stride; a.p_stride = p_stride; a.q_stride = q_stride;
         a.sing = s->d_sing_bits; a.grad = grad_3xv; a.V = V; a.T = T; a.nf = nf;
         fill_freqs(a.fq, k_re, f0, nf);
-        const size_t smem = sizeof(float) * (size_t)nf * (6 * kBwdTest * 2 + 6 * kBwdTrial * 2 + kBwdTrial * 2);
+        return a;
+    };
+    for (int f0 = 0; f0 < n_freq; f0 += kBwdMaxF) {
+        const int nf = std::min(kBwdMaxF, n_freq - f0);
+        const BwdArgs a = args(f0, nf);
+        const size_t smem = sizeof(float) * (size_t)((nf + 1) / 2) * 4 * (6 * kBwdTest + 6 * kBwdTrial + kBwdTrial);
         dim3 grid((T + kBwdTrial - 1) / kBwdTrial, (T + kBwdTest - 1) / kBwdTest);
         k_asm_bwd<<<grid, kBwdThreads, smem, st>>>(a);
         HBEM_LAUNCH_CHECK("k_asm_bwd");
+    }
+    for (int f0 = 0; f0 < n_freq; f0 += kBwdTouchF) {
+        const BwdArgs a = args(f0, std::min(kBwdTouchF, n_freq - f0));
         if (s->n_pairs > 0) {
             DuffyBwdArgs d{};
             d.b = a; d.pairs = s->d_pairs; d.rule = s->d_rule; d.rule_w = s->d_rule_w; d.n_pairs = s->n_pairs;

@@ -1,0 +1,48 @@
+"""Assembly gradients over more frequencies than one launch stages, and an odd count, against one frequency a call.
+
+Tolerance 2e-5 relative: a launch's FP32 sums over the frequencies are rounded per term (2^-24), and the touching
+pairs' lane sums cancel by up to two orders of magnitude (2^-24 * 100 = 6e-6) in either grouping."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+if not torch.cuda.is_available():  # pragma: no cover - CPU containers
+    pytest.skip("needs a CUDA device", allow_module_level=True)
+
+from hornlab_metal_bem_b200 import generators as G  # noqa: E402
+from hornlab_metal_bem_b200.geometry import build_geometry_buffers  # noqa: E402
+from hornlab_metal_bem_b200.mesh import make_pure_function_spaces  # noqa: E402
+from hornlab_metal_bem_b200.native import NativeSession, _np_ptr, _stream_ptr, _t_ptr, check  # noqa: E402
+
+
+@pytest.mark.parametrize("freqs", [1, 2, 3, 21])
+@pytest.mark.parametrize("level", [0, 1])
+def test_assembly_gradient_sums_over_frequencies(freqs, level):
+    mesh = G.icosphere(level, 0.1)   # 20 triangles: less than a tile; 80: ragged
+    p1, dp0 = make_pure_function_spaces(mesh.grid)
+    b = build_geometry_buffers(mesh.grid, mesh.physical_tags, p1, dp0)
+    n, T, V = b.p1_dof_count, b.n_triangles, np.asarray(b.vertices_3xn_f32).shape[1]
+    rng = np.random.default_rng(freqs)
+    k = np.linspace(5.0, 60.0, freqs).astype(np.float32)
+    dev = torch.device("cuda")
+    lam, p = (torch.tensor(rng.standard_normal((2, freqs, n)), dtype=torch.float32, device=dev) for _ in range(2))
+    q = torch.tensor(rng.standard_normal((2, freqs, T)), dtype=torch.float32, device=dev)
+    q[:, :, T // 2:] = 0.0
+    with NativeSession(b, check_open_edges=False) as s:
+        def grad(f0, f1):
+            out = torch.zeros((3, V), dtype=torch.float64, device=dev)
+            cut = [x[f0:f1].contiguous() for z in (lam, p, q) for x in z]
+            kk = np.ascontiguousarray(k[f0:f1])
+            check(s.lib.hbem_assemble_backward(
+                s.handle, f1 - f0, _np_ptr(kk), None, _t_ptr(cut[0]), _t_ptr(cut[1]), n, _t_ptr(cut[2]), _t_ptr(cut[3]),
+                n, _t_ptr(cut[4]), _t_ptr(cut[5]), T, _t_ptr(out), _stream_ptr()), "hbem_assemble_backward")
+            torch.cuda.synchronize()
+            return out.cpu().numpy()
+
+        whole = grad(0, freqs)
+        single = sum(grad(f, f + 1) for f in range(freqs))
+    assert np.linalg.norm(whole - single) <= 2e-5 * np.linalg.norm(single)
