@@ -3,10 +3,14 @@
 //   p(x_o) = sum_tri sum_q w_q 2|tau| sum_images [dG/dn_y(x_o, y_q) p(y_q) - G(x_o, y_q) q_tri]
 //   (reference evaluate_field_regular, main.swift:4135-4203; real k only, as there)
 //
-// One CTA per (frequency, tile of 8 observation points); threads stride over
-// triangles, interpolate the P1 pressure to the 6 quadrature points once per
-// triangle, and accumulate the 8 observation sums in registers before a block
-// reduction.  Tag averages (main.swift:807-841) use FP64 block sums.
+// One CTA per (frequency, tile of 8 observation points, 2 where the grid would
+// leave SMs idle); threads stride over triangles, interpolate the P1 pressure
+// to the 6 quadrature points once per triangle, and accumulate the tile's
+// observation sums in registers before a block reduction (the same order of
+// sums for either tile).  111 points at one frequency on the quarter horn of
+// 1950 triangles are 14 CTAs of 8 points (373 us) or 56 of 2 (60 us); from 296
+// CTAs of 8 on, two per SM, the larger tile shares more of the interpolation.
+// Tag averages (main.swift:807-841) use FP64 block sums.
 //
 // Phase accuracy: at 2 m and 20 kHz, k r is ~730 rad, so an FP32 distance
 // (relative error ~6e-8) alone puts ~4e-5 rad into the phase, which the sum
@@ -26,7 +30,6 @@
 namespace hbem {
 namespace {
 
-constexpr int kObsTile = 8;
 constexpr int kFieldThreads = 256;
 
 struct FieldArgs {
@@ -80,7 +83,7 @@ __device__ __forceinline__ void fsample(double yx, double yy, double yz, double 
     ai += dre * pi + dim * pr - (gc * qi + gs * qr);
 }
 
-template <int SYM>
+template <int SYM, int kObsTile>
 __global__ void __launch_bounds__(kFieldThreads, 2) k_field(const __grid_constant__ FieldArgs a) {
     __shared__ double s_obs[kObsTile][3];
     __shared__ float s_obsf[kObsTile][3];
@@ -165,6 +168,18 @@ __global__ void __launch_bounds__(kFieldThreads, 2) k_field(const __grid_constan
     }
 }
 
+template <int TILE>
+void launch_field_t(int sym, const FieldArgs &a, int nf, cudaStream_t st) {
+    const dim3 grid((a.n_obs + TILE - 1) / TILE, nf);
+    switch (sym) {
+        case 0: k_field<0, TILE><<<grid, kFieldThreads, 0, st>>>(a); break;
+        case 1: k_field<1, TILE><<<grid, kFieldThreads, 0, st>>>(a); break;
+        case 2: k_field<2, TILE><<<grid, kFieldThreads, 0, st>>>(a); break;
+        case 3: k_field<3, TILE><<<grid, kFieldThreads, 0, st>>>(a); break;
+        default: k_field<4, TILE><<<grid, kFieldThreads, 0, st>>>(a); break;
+    }
+}
+
 __global__ void k_tag_avg(const int *__restrict__ tags, const float *__restrict__ areas, const int *__restrict__ l2g,
                           const float *p_re, const float *p_im, long long p_stride, int T, const int *__restrict__ want,
                           double *out, int n_tags) {
@@ -218,14 +233,8 @@ int launch_field(Session &s, int n_freq, const float *k_re, const float *p_re, c
             a.k[f] = k_re[f0 + f];
             a.kt[f] = (double)k_re[f0 + f] / (2.0 * 3.14159265358979323846);
         }
-        dim3 grid((n_obs + kObsTile - 1) / kObsTile, nf);
-        switch (s.sym) {
-            case 0: k_field<0><<<grid, kFieldThreads, 0, st>>>(a); break;
-            case 1: k_field<1><<<grid, kFieldThreads, 0, st>>>(a); break;
-            case 2: k_field<2><<<grid, kFieldThreads, 0, st>>>(a); break;
-            case 3: k_field<3><<<grid, kFieldThreads, 0, st>>>(a); break;
-            default: k_field<4><<<grid, kFieldThreads, 0, st>>>(a); break;
-        }
+        if ((n_obs + 7) / 8 * nf < 2 * 148) launch_field_t<2>(s.sym, a, nf, st);
+        else launch_field_t<8>(s.sym, a, nf, st);
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return cuda_fail(e, "k_field launch");
         count_launch();
