@@ -2,8 +2,8 @@
 // batched over matrices.  K = 16/32 inside a block column, 64 for the
 // block's trailing matrix.
 //
-// CUDA-core path: 64 x 64 complex output tile per 256-thread CTA, 4 x 4
-// complex outputs per thread, L and U chunks staged in shared memory by
+// CUDA-core path: 64 x 64 (or 32 x 64) complex output tile per 256-thread CTA,
+// 4 x 4 (2 x 4) complex outputs per thread, L and U chunks staged in shared memory by
 // double-buffered cp.async and read with 128-bit broadcast loads; FP32 FMA gives the exact-FP32 products of
 // LAPACK cgemm-based cgetrf.
 #include <cuda.h>
@@ -20,29 +20,30 @@ struct TcWorkspace;
 namespace {
 
 // C[start:n, col_start:col_end] -= L[start:n, k0:k0+kw] * U[k0:k0+kw, col_start:col_end]
-// (kw a multiple of 16) for one 64 x 64 complex tile per CTA, K in chunks of
+// (kw a multiple of 16) for one TM x 64 complex tile per CTA, K in chunks of
 // 16 double-buffered through cp.async (the next chunk's loads
 // are in flight while the current one is multiplied); 4 x 4 complex
 // accumulators per thread.  L is stored transposed ([k][row]) with the row
 // index XOR-swizzled by k, so the coalesced row-segment loads do not all
 // land on one bank.
+template <int TM>
 __global__ void __launch_bounds__(256) k_trailing_simt(float *a_re, float *a_im, long long lda, long long a_stride,
                                                        int n, int k0, int kw, int start, int col_start, int col_end) {
-    constexpr int KC = 16;
-    __shared__ __align__(16) float Lr[2][KC][64], Li[2][KC][64];
+    constexpr int KC = 16, RM = TM / 16;   // rows per thread
+    __shared__ __align__(16) float Lr[2][KC][TM], Li[2][KC][TM];
     __shared__ __align__(16) float Ur[2][KC][64], Ui[2][KC][64];
     const int mat = blockIdx.z;
     float *are = a_re + (size_t)mat * a_stride, *aim = a_im + (size_t)mat * a_stride;
-    const int row0 = start + blockIdx.y * 64, col0 = col_start + blockIdx.x * 64;
+    const int row0 = start + blockIdx.y * TM, col0 = col_start + blockIdx.x * 64;
     const int tid = threadIdx.x;
     const int tx = tid & 15, ty = tid >> 4;
-    float cr[4][4], ci[4][4];
+    float cr[RM][4], ci[RM][4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < RM; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j) cr[i][j] = ci[i][j] = 0.f;
     auto load_chunk = [&](int kc, int sbuf) {
-        for (int e = tid; e < 64 * KC; e += 256) {
+        for (int e = tid; e < TM * KC; e += 256) {
             const int r = e / KC, kk = e - r * KC;
             const int gr = row0 + r;
             const bool ok = gr < n;
@@ -73,15 +74,24 @@ __global__ void __launch_bounds__(256) k_trailing_simt(float *a_re, float *a_im,
         __syncthreads();
 #pragma unroll
         for (int kk = 0; kk < KC; ++kk) {
-            const int lo = (ty * 4) ^ ((kk & 7) << 2);   // XOR of a multiple of 4 keeps the float4 whole
-            const float4 lr = *reinterpret_cast<const float4 *>(&Lr[sbuf][kk][lo]);
-            const float4 li = *reinterpret_cast<const float4 *>(&Li[sbuf][kk][lo]);
+            const int lo = (ty * RM) ^ ((kk & 7) << 2);   // XOR of a multiple of 4 keeps the vector whole
+            float a_r[RM], a_i[RM];
+            if constexpr (RM == 4) {
+                const float4 lr = *reinterpret_cast<const float4 *>(&Lr[sbuf][kk][lo]);
+                const float4 li = *reinterpret_cast<const float4 *>(&Li[sbuf][kk][lo]);
+                a_r[0] = lr.x; a_r[1] = lr.y; a_r[2] = lr.z; a_r[3] = lr.w;
+                a_i[0] = li.x; a_i[1] = li.y; a_i[2] = li.z; a_i[3] = li.w;
+            } else {
+                const float2 lr = *reinterpret_cast<const float2 *>(&Lr[sbuf][kk][lo]);
+                const float2 li = *reinterpret_cast<const float2 *>(&Li[sbuf][kk][lo]);
+                a_r[0] = lr.x; a_r[1] = lr.y;
+                a_i[0] = li.x; a_i[1] = li.y;
+            }
             const float4 ur = *reinterpret_cast<const float4 *>(&Ur[sbuf][kk][tx * 4]);
             const float4 ui = *reinterpret_cast<const float4 *>(&Ui[sbuf][kk][tx * 4]);
-            const float a_r[4] = {lr.x, lr.y, lr.z, lr.w}, a_i[4] = {li.x, li.y, li.z, li.w};
             const float b_r[4] = {ur.x, ur.y, ur.z, ur.w}, b_i[4] = {ui.x, ui.y, ui.z, ui.w};
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
+            for (int i = 0; i < RM; ++i)
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     cr[i][j] = fmaf(a_r[i], b_r[j], cr[i][j]);
@@ -94,8 +104,8 @@ __global__ void __launch_bounds__(256) k_trailing_simt(float *a_re, float *a_im,
         sbuf ^= 1;
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int gr = row0 + ty * 4 + i;
+    for (int i = 0; i < RM; ++i) {
+        const int gr = row0 + ty * RM + i;
         if (gr >= n) continue;
         const int gc = col0 + tx * 4;
         float *pr = are + (size_t)gr * lda + gc;
@@ -130,8 +140,17 @@ int launch_trailing_simt(int n, int batch, int k0, int kw, int start, int col_st
     const int m = n - start, w = col_end - col_start;
     if (m <= 0 || w <= 0) return HBEM_OK;
     if (kw % 16) return fail(HBEM_ERR_ARG, "trailing update: K must be a multiple of 16");
-    dim3 grid((w + 63) / 64, (m + 63) / 64, batch);
-    k_trailing_simt<<<grid, 256, 0, st>>>(a_re, a_im, lda, a_stride, n, k0, kw, start, col_start, col_end);
+    // tiles of 32 rows while 64-row ones leave SMs idle (a look-ahead block of
+    // 64 columns at n = 1043, one matrix: 16 CTAs of 64; the same sums in the
+    // same order): factorisation of 642 x 8 1266 -> 1228 us, 1043 x 1 2122 -> 2098
+    const long long tiles = (long long)((w + 63) / 64) * ((m + 63) / 64) * batch;
+    if (tiles < 148) {
+        const dim3 grid((w + 63) / 64, (m + 31) / 32, batch);
+        k_trailing_simt<32><<<grid, 256, 0, st>>>(a_re, a_im, lda, a_stride, n, k0, kw, start, col_start, col_end);
+    } else {
+        const dim3 grid((w + 63) / 64, (m + 63) / 64, batch);
+        k_trailing_simt<64><<<grid, 256, 0, st>>>(a_re, a_im, lda, a_stride, n, k0, kw, start, col_start, col_end);
+    }
     HBEM_LAUNCH_CHECK("k_trailing_simt");
     return HBEM_OK;
 }
