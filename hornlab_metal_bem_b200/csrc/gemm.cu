@@ -173,26 +173,30 @@ int launch_trailing_update(int n, int batch, int k0, int kw, int start, int col_
 // products: each split keeps 11 significant bits, so hi + lo carries 22 and
 // the dropped lo x lo term is below 2^-22 of the product) for the plain LU.
 //
-// The complex update C -= L U is one real GEMM: for a tile of 64 complex rows
-// the 128 MMA rows are [Lr, -Li] (real part) and [Li, Lr] (imaginary part)
-// against B = [Ur; Ui] (K = 2 x 64).  Each FP32 operand x is split into
-// hi = bf16(x) and lo = bf16(x - hi); A B ~ Ah Bh + Ah Bl + Al Bh.  The packed
-// operands hold each split once, A2 = [Ah | Al] and B2^T = [Bh | Bl] (both
-// K-major, 256 elements per row, written by k_pack_*); the three products are
-// three MMA groups over the same shared-memory blocks.  A CTA takes work units
-// of consecutive column tiles of one row block and keeps that row block's A2
-// resident in shared memory while B2 streams through a ring (k_trailing_tc:
+// Each FP32 operand x is split into hi = bf16(x) (or tf32(x)) and lo of the
+// rest; A B ~ Ah Bh + Ah Bl + Al Bh.  The packed operands hold each split once
+// (K-major rows [hi | lo], written by k_pack_*); the three products are three
+// MMA groups over the same shared-memory blocks.  A CTA takes work units of
+// consecutive column tiles of one row block and keeps that row block's A
+// resident in shared memory while B streams through a ring (k_trailing_tc:
 // TMA, single-thread MMA issue into two FP32 TMEM accumulators, C staged
-// through shared memory by the epilogue warps).  Per variant (the same 224 KB
-// of shared memory):
-//   BF16x3: tiles of 64 complex rows x 64 columns, A2 64 KB (4 K-blocks of
-//           128 bytes per row), ring of 6 x 16 KB, two 32 KB C tiles;
-//   TF32x3 with K = 64 (and BF16x3 with K = 128): tiles of 64 complex rows x
-//           32 columns, A2 128 KB (8 K-blocks), ring of 6 x 8 KB, three
-//           16 KB C tiles (C prefetched two tiles ahead);
-//   TF32x3 with K = 32 (two passes per 64-column LU block): the BF16x3
-//           K = 64 shape (A2 64 KB, 64-column tiles, 6 x 16 KB ring, two
-//           32 KB C tiles).
+// through shared memory by the epilogue warps).
+//   BF16x3: one real GEMM.  The 128 MMA rows of 64 complex rows are [Lr, -Li]
+//           (real part) and [Li, Lr] (imaginary part) against B = [Ur; Ui], K =
+//           2 x 64: tiles of 64 complex columns, A 64 KB, ring of 6 x 16 KB, two
+//           32 KB C tiles.  With K = 2 x 128 tiles of 32 columns, A 128 KB, ring
+//           of 6 x 8 KB, three 16 KB C tiles (prefetched two tiles ahead).
+//   TF32x3: operands twice as wide, so the four real products are kept apart:
+//           MMA rows [Lr; Li], MMA columns [Ur | Ui] (N = 128), K = 64, and the
+//           epilogue combines Lr Ur, Li Ui, Lr Ui and Li Ur in the C tile.  A
+//           row block is 64 KB instead of 128 KB for the same MMA work: tiles
+//           of 64 complex columns, ring of 3 x 32 KB, two 32 KB C tiles.  The
+//           [Lr, -Li] form fits this memory at K = 32 only, so it read, packed
+//           and wrote C twice per 64-column block; the whole factorisation
+//           took (two K = 32 passes -> this) 1043 x 40 4.75 -> 3.72 ms, 1900 x
+//           20 10.2 -> 7.6, 4217 x 2 14.6 -> 12.0, 4217 x 6 27.6 -> 19.7, 8000 x
+//           2 59 -> 45, 14 000 x 1 152 -> 115 ms.  Bound by the tensor pipe's
+//           TF32 rate and C's read-modify-write together.
 // Every mbarrier wait is bounded; a timeout sets the status word and the CTA
 // returns after releasing its TMEM.
 // ===========================================================================
@@ -208,18 +212,19 @@ constexpr long long kSpinLimit = 1LL << 24;
 // of one update (64: one LU block; 128: two blocks, BF16x3 only).
 template <bool TF32, int KC>
 struct TcCfg {
-    static_assert(KC == 64 || (KC == 128 && !TF32) || (KC == 32 && TF32),
-                  "tensor-core update: K = 64, 128 with BF16x3, or 32 with TF32x3");
+    static_assert(KC == 64 || (KC == 128 && !TF32), "tensor-core update: K = 64, or 128 with BF16x3");
+    static constexpr bool Apart = TF32;                // the four real products apart
     static constexpr int ES = TF32 ? 4 : 2;            // operand bytes
     static constexpr int EPB = 128 / ES;               // operand elements per 128-byte K-block
-    static constexpr int K2 = 4 * KC;                  // packed elements per row: hi (real K = 2 KC), lo
-    static constexpr int KBH = 2 * KC / EPB;           // K-blocks of one split
-    static constexpr int N = KBH == 4 ? 32 : 64;       // columns per tile
-    static constexpr int ABytes = 2 * KBH * kTcABlk;   // resident A2 of a row block
-    static constexpr int BBlk = N * 128;               // one B K-block
+    static constexpr int KS = Apart ? KC : 2 * KC;     // packed elements of one split: real K
+    static constexpr int K2 = 2 * KS;                  // packed elements per row: hi, lo
+    static constexpr int KBH = KS / EPB;               // K-blocks of one split
+    static constexpr int N = KBH == 4 ? 32 : 64;       // complex columns per tile
+    static constexpr int BN = Apart ? 2 * N : N;       // MMA columns: packed B rows per tile
+    static constexpr int ABytes = 2 * KBH * kTcABlk;   // resident A of a row block
+    static constexpr int BBlk = BN * 128;              // one B K-block
     static constexpr int StageBytes = 2 * BBlk;        // ring stage: Bh and Bl of one K-block
-    // B ring: one and a half 32-column tiles (K-block 4) / three 64-column tiles ahead
-    static constexpr int Stages = 6;
+    static constexpr int Stages = Apart ? 3 : 6;       // one and a half tiles ahead (three of BF16x3's K = 64)
     static constexpr int CBytes = kTcM * N * 4;        // one C tile staged in shared memory
     // C buffers: the 32-column tiles prefetch C two tiles ahead (one tile's
     // time is shorter than the HBM latency of its C), the 64-column ones one
@@ -227,7 +232,7 @@ struct TcCfg {
     static constexpr int Fmt = TF32 ? 2 : 1;           // instruction-descriptor operand format
     static constexpr size_t Smem =
         (size_t)ABytes + (size_t)Stages * StageBytes + (size_t)CBufs * CBytes + 1024;
-    static_assert(Smem <= 227 * 1024, "tensor-core trailing update: shared memory");
+    static_assert(Smem <= 226 * 1024, "tensor-core trailing update: shared memory");
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {
@@ -349,7 +354,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_trailing_tc(const __grid_cons
                                                                 int chunk, int n_units, int *status) {
     using Cfg = TcCfg<TF32, KC>;
     constexpr int kTcN = Cfg::N, kTcStages = Cfg::Stages, kTcStageBytes = Cfg::StageBytes, kTcABytes = Cfg::ABytes;
-    constexpr int KBH = Cfg::KBH, EPB = Cfg::EPB;
+    constexpr int KBH = Cfg::KBH, EPB = Cfg::EPB, BN = Cfg::BN;
+    constexpr int BRows = BN / kTcN;   // packed B rows per column
     extern __shared__ uint8_t s_raw[];
     __shared__ uint64_t s_full[kTcStages], s_empty[kTcStages];
     __shared__ uint64_t s_acc_full[2], s_acc_empty[2];
@@ -379,7 +385,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_trailing_tc(const __grid_cons
     }
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)),
-                     "r"(2 * kTcN));
+                     "r"(2 * BN));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -418,7 +424,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_trailing_tc(const __grid_cons
                 }
                 bool last;
                 do {
-                    const int row_b = w.mat * cols_pad + w.tn * kTcN;
+                    const int row_b = BRows * (w.mat * cols_pad + w.tn * kTcN);
                     for (int kh = 0; kh < KBH; ++kh, ++g) {
                         const int s = (int)(g % kTcStages);
                         const int u = (int)(g / kTcStages);
@@ -457,7 +463,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_trailing_tc(const __grid_cons
     } else if (warp == 0) {
         // ---- MMA issuer
         if (lane == 0) {
-            constexpr uint32_t idesc = umma_idesc(kTcM, kTcN, Cfg::Fmt);
+            constexpr uint32_t idesc = umma_idesc(kTcM, BN, Cfg::Fmt);
             bool ok = true;
             long long g = 0;
             int i = 0;        // tiles
@@ -475,7 +481,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_trailing_tc(const __grid_cons
                         break;
                     }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint32_t acc_addr = tmem + (uint32_t)(b * kTcN);
+                    const uint32_t acc_addr = tmem + (uint32_t)(b * BN);
                     for (int kh = 0; kh < KBH; ++kh, ++g) {
                         const int s = (int)(g % kTcStages);
                         const int u = (int)(g / kTcStages);
@@ -609,36 +615,50 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_trailing_tc(const __grid_cons
                 const int r = q * 32 + lane;
                 const int c0 = HALF * h;
                 uint32_t v[HALF];
-                const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * kTcN + c0);
-                if constexpr (HALF == 32)
-                    asm volatile(
-                        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, "
-                        "%12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, "
-                        "%30, %31}, [%32];"
-                        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
-                          "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]),
-                          "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]),
-                          "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]),
-                          "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-                        : "r"(taddr));
-                else
-                    asm volatile(
-                        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, "
-                        "%12, %13, %14, %15}, [%16];"
-                        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
-                          "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]),
-                          "=r"(v[14]), "=r"(v[15])
-                        : "r"(taddr));
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                auto load = [&](uint32_t taddr) {
+                    if constexpr (HALF == 32)
+                        asm volatile(
+                            "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, "
+                            "%12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, "
+                            "%30, %31}, [%32];"
+                            : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
+                              "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]),
+                              "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]),
+                              "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]),
+                              "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+                            : "r"(taddr));
+                    else
+                        asm volatile(
+                            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, "
+                            "%12, %13, %14, %15}, [%16];"
+                            : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
+                              "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]),
+                              "=r"(v[14]), "=r"(v[15])
+                            : "r"(taddr));
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                };
+                // C row r of the staged tile (real rows, then imaginary ones) plus s times the loaded columns
+                auto add = [&](int row, float s) {
 #pragma unroll
-                for (int jj = 0; jj < HALF / 4; ++jj) {
-                    float4 *p4 = reinterpret_cast<float4 *>(sC + sidx(r, c0 + 4 * jj));
-                    float4 cv = *p4;
-                    cv.x -= __uint_as_float(v[4 * jj]);
-                    cv.y -= __uint_as_float(v[4 * jj + 1]);
-                    cv.z -= __uint_as_float(v[4 * jj + 2]);
-                    cv.w -= __uint_as_float(v[4 * jj + 3]);
-                    *p4 = cv;
+                    for (int jj = 0; jj < HALF / 4; ++jj) {
+                        float4 *p4 = reinterpret_cast<float4 *>(sC + sidx(row, c0 + 4 * jj));
+                        float4 cv = *p4;
+                        cv.x = fmaf(s, __uint_as_float(v[4 * jj]), cv.x);
+                        cv.y = fmaf(s, __uint_as_float(v[4 * jj + 1]), cv.y);
+                        cv.z = fmaf(s, __uint_as_float(v[4 * jj + 2]), cv.z);
+                        cv.w = fmaf(s, __uint_as_float(v[4 * jj + 3]), cv.w);
+                        *p4 = cv;
+                    }
+                };
+                const uint32_t tadr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * BN + c0);
+                load(tadr);
+                add(r, -1.f);
+                if constexpr (Cfg::Apart) {
+                    // so far re -= Lr Ur and im -= Li Ur; now im -= Lr Ui, re += Li Ui: the rows
+                    // another warp has just finished
+                    load(tadr + kTcN);
+                    epi_bar();
+                    add(r ^ 64, r < 64 ? -1.f : 1.f);
                 }
             }
             // hand the accumulator back (one arrival per warp)
@@ -678,7 +698,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_trailing_tc(const __grid_cons
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * kTcN));
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * BN));
 }
 
 // Operand splits: hi = x rounded to the operand format, lo = (x - hi) rounded
@@ -712,7 +732,8 @@ struct TcSplit<true> {
 };
 
 // Pack L21 (rows start..n, cols k0..k0+KC) into A2 (K-major, hi/lo splits):
-// real-part row [Lr | -Li], imaginary-part row [Li | Lr], hi then lo.
+// real-part row [Lr | -Li], imaginary-part row [Li | Lr] (rows Lr and Li where
+// the products are kept apart), hi then lo.
 template <bool TF32, int KC>
 __global__ void k_pack_a(const float *a_re, const float *a_im, long long lda, long long a_stride, int n, int start,
                          int k0, int rows3, int rows_used, typename TcSplit<TF32>::T *A2) {
@@ -735,16 +756,20 @@ __global__ void k_pack_a(const float *a_re, const float *a_im, long long lda, lo
     auto put = [](T *row, int k2, float x) {
         const T h = S::hi(x);
         row[k2] = h;
-        row[2 * KC + k2] = S::hi(x - S::val(h));
+        row[TcCfg<TF32, KC>::KS + k2] = S::hi(x - S::val(h));
     };
     put(re_row, k, lr);
-    put(re_row, KC + k, -li);
     put(im_row, k, li);
-    put(im_row, KC + k, lr);
+    if constexpr (!TcCfg<TF32, KC>::Apart) {
+        put(re_row, KC + k, -li);
+        put(im_row, KC + k, lr);
+    }
 }
 
 // Pack U12 (rows k0..k0+KC, cols start..col_end) into B2^T (K-major, hi/lo
-// splits): per column [hi Ur | hi Ui | lo Ur | lo Ui], KC entries each.
+// splits): per column [hi Ur | hi Ui | lo Ur | lo Ui], KC entries each; where
+// the products are kept apart, rows [hi Ur | lo Ur] of a tile's 64 columns,
+// then its rows [hi Ui | lo Ui].
 template <bool TF32, int KC>
 __global__ void __launch_bounds__(256) k_pack_b(const float *a_re, const float *a_im, long long lda,
                                                 long long a_stride, int start, int col_end, int k0, int cols_pad,
@@ -786,7 +811,11 @@ __global__ void __launch_bounds__(256) k_pack_b(const float *a_re, const float *
                 v0 = S::hi(x0 - S::val(v0));
                 v1 = S::hi(x1 - S::val(v1));
             }
-            S::store2(B2 + ((size_t)mat * cols_pad + j) * K2 + part * KC + kc + k, v0, v1);
+            if constexpr (TcCfg<TF32, KC>::Apart)
+                S::store2(B2 + (2 * ((size_t)mat * cols_pad + j0) + (part & 1) * 64 + jj) * K2 + (part >> 1) * KC + kc + k,
+                          v0, v1);
+            else
+                S::store2(B2 + ((size_t)mat * cols_pad + j) * K2 + part * KC + kc + k, v0, v1);
         }
     }
 }
@@ -830,8 +859,7 @@ int make_map(CUtensorMap *map, void *ptr, long long rows, int box_rows, int es, 
 // Packed-operand workspace and tensor maps for one factorisation: sized for
 // the first (largest) trailing update and reused by the later, smaller ones.
 // tf32: TF32x3 operands (plain LU) instead of BF16x3 (mixed LU); kc: the
-// complex K of one update (64; 128 for BF16x3; 32 for TF32x3, two passes per
-// 64-column block).
+// complex K of one update (64; 128 for BF16x3).
 struct TcWorkspace {
     void *A2 = nullptr, *B2 = nullptr;
     int rows3 = 0, cols_pad = 0, batch = 0, kc = 64;
@@ -841,25 +869,27 @@ struct TcWorkspace {
 
 int tc_workspace_create(int n, int batch, bool tf32, int kc, TcWorkspace **out, cudaStream_t st) {
     *out = nullptr;
-    if (!(kc == 64 || (kc == 128 && !tf32) || (kc == 32 && tf32)))
-        return fail(HBEM_ERR_ARG, "tensor-core update: K = 64, 128 with BF16x3, or 32 with TF32x3");
+    if (!(kc == 64 || (kc == 128 && !tf32)))
+        return fail(HBEM_ERR_ARG, "tensor-core update: K = 64, or 128 with BF16x3");
     auto *w = new TcWorkspace();
-    const int es = tf32 ? 4 : 2, k2 = 4 * kc;
-    const int tn = 2 * kc * es / 128 == 4 ? 32 : 64;   // the configuration's tile width (TcCfg::N)
+    // the configuration's operand bytes, packed row, tile width, MMA columns per tile and packed B rows per column
+    const int es = tf32 ? 4 : 2, k2 = tf32 ? TcCfg<true, 64>::K2 : 4 * kc;
+    const int tn = kc == 128 ? TcCfg<false, 128>::N : 64;
+    const int bn = tf32 ? TcCfg<true, 64>::BN : tn, b_rows = bn / tn;
     w->tf32 = tf32;
     w->kc = kc;
     w->rows3 = ((n + 63) / 64) * kTcM;
     w->cols_pad = ((n + tn - 1) / tn) * tn;
     w->batch = batch;
     cudaError_t e = cudaMallocAsync(&w->A2, (size_t)batch * w->rows3 * k2 * es, st);
-    if (e == cudaSuccess) e = cudaMallocAsync(&w->B2, (size_t)batch * w->cols_pad * k2 * es, st);
+    if (e == cudaSuccess) e = cudaMallocAsync(&w->B2, (size_t)batch * w->cols_pad * b_rows * k2 * es, st);
     if (e != cudaSuccess) {
         if (w->A2) cudaFreeAsync(w->A2, st);
         delete w;
         return cuda_fail(e, "tensor-core workspace");
     }
     int rc = make_map(&w->ma, w->A2, (long long)batch * w->rows3, kTcM, es, k2);
-    if (rc == HBEM_OK) rc = make_map(&w->mb, w->B2, (long long)batch * w->cols_pad, tn, es, k2);
+    if (rc == HBEM_OK) rc = make_map(&w->mb, w->B2, (long long)batch * w->cols_pad * b_rows, bn, es, k2);
     if (rc != HBEM_OK) {
         cudaFreeAsync(w->A2, st);
         cudaFreeAsync(w->B2, st);
@@ -877,9 +907,8 @@ void tc_workspace_destroy(TcWorkspace *w, cudaStream_t st) {
     delete w;
 }
 
-// The K one launch_trailing_tc call consumes: the workspace's K, or 64 for
-// the TF32x3 K = 32 workspace, which runs two passes per call.
-int tc_workspace_k(const TcWorkspace *w) { return w ? (w->tf32 && w->kc == 32 ? 64 : w->kc) : 0; }
+// The K one launch_trailing_tc call consumes
+int tc_workspace_k(const TcWorkspace *w) { return w ? w->kc : 0; }
 
 namespace {
 
@@ -942,15 +971,6 @@ int launch_trailing_tc(TcWorkspace *w, int n, int batch, int k0, int start, int 
                        float *a_im, long long lda, long long a_stride, int *status, cudaStream_t st,
                        int reserve_sms) {
     if (n - start <= 0 || col_end - col_start <= 0) return HBEM_OK;
-    if (w->tf32 && w->kc == 32) {
-        // the 64 columns of an LU block as two K = 32 passes (C read and
-        // written twice, each pass in the 64 KB-A, 64-column-tile shape)
-        int rc = launch_trailing_tc_t<true, 32>(w, n, batch, k0, start, col_start, col_end, a_re, a_im, lda,
-                                                a_stride, status, st, reserve_sms);
-        if (rc != HBEM_OK) return rc;
-        return launch_trailing_tc_t<true, 32>(w, n, batch, k0 + 32, start, col_start, col_end, a_re, a_im, lda,
-                                              a_stride, status, st, reserve_sms);
-    }
     if (w->tf32)
         return launch_trailing_tc_t<true, 64>(w, n, batch, k0, start, col_start, col_end, a_re, a_im, lda, a_stride,
                                               status, st, reserve_sms);
