@@ -2,7 +2,13 @@
 // replacing LAPACK cgesv/cgetrf/cgetrs (reference main.swift:7834-7941,
 // 8015-8020).  Matrices are planar (re, im) float32, row-major.
 //
-// Two-level right-looking blocked factorisation, batched over matrices:
+// Two-level right-looking blocked factorisation, batched over matrices.
+// Refined factorisations (HBEM_PREC_TF32X3, HBEM_PREC_MIXED), per 64-column
+// block of at most 6144 rows:
+//     k_panel_block  : the whole block in one CTA or cluster, rows in place;
+//     k_move_solve   : its net row moves and U12 = L11^-1 A12;
+//     trailing       : A22 -= L21 U12 with K = 64.
+// HBEM_PREC_PLAIN, taller blocks and the HBEM_TUNE_LU_PANEL widths:
 //   for each 64-column block b0:
 //     for each inner sub-panel c (64, 32 or 16 columns):
 //       k_panel      : factor rows c..n of the sub-panel with partial pivoting
@@ -15,9 +21,10 @@
 //     k_swap_trsm    : the block's 64 swaps on all other columns and the
 //                      64-row TRSM U12 = L11^-1 A12;
 //     trailing       : A22 -= L21 U12 with K = 64.
-// The solve applies the pivots then runs blocked forward / backward
-// substitution: op(A) = A with n > 128 in 128-row block steps over many CTAs
-// (k_trsv_*), A^T / A^H and small n in one CTA per right-hand side (k_getrs).
+// The solve applies the pivots then runs the two triangular phases: n <= 128 in
+// one CTA per right-hand side (k_getrs), else a wavefront of one CTA per 32-row
+// block, a launch per phase (k_trsv_wave) or, in refinement and the condition
+// estimate, one for both (k_trsv_both).
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 

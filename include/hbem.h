@@ -101,14 +101,19 @@ long long hbem_launch_count(void);
  *                            one CTA holds it, else 32 where one CTA holds
  *                            it, else 16 where one CTA holds it, else 32 in
  *                            a cluster; 64: as 0, but the whole block also
- *                            in an 8-CTA cluster where that holds it)
+ *                            in an 8-CTA cluster where that holds it).  With
+ *                            0, HBEM_PREC_TF32X3 and HBEM_PREC_MIXED factor
+ *                            whole 64-column blocks of up to 6144 rows in one
+ *                            launch instead
  *   HBEM_TUNE_LU_SOLVE:      triangular solves (1: one CTA per right-hand
  *                            side, 2: blocked multi-CTA steps, 3: wavefront,
  *                            one CTA per 32-row block; 0: one CTA per
- *                            right-hand side for n <= 128, else wavefront)
+ *                            right-hand side for n <= 128, else wavefront,
+ *                            refinement and condition estimate with both
+ *                            triangular phases in one launch up to n = 25600)
  *   HBEM_TUNE_ASM_PAIRS:     regular assembly (0: unordered pairs, both
- *                            orders from one kernel evaluation; 1: ordered
- *                            pairs, two wavenumbers per evaluation)
+ *                            orders and two wavenumbers from one kernel
+ *                            evaluation; 1: ordered pairs, two wavenumbers)
  *   HBEM_TUNE_DUFFY:         singular corrections (1: one wavenumber per
  *                            warp, 2: two wavenumbers per warp)
  *   HBEM_TUNE_LU_LOOKAHEAD:  LU schedule (0: look-ahead, the block after
@@ -136,7 +141,9 @@ long long hbem_launch_count(void);
  *                            built-in 128 for n > 16000, else 64); the FP32
  *                            LU's TF32x3 bulk takes K = 64 with any value
  *   HBEM_TUNE_LU_PANEL_KERNEL: sub-panels with their rows in shared memory
- *                            (0, built-in) or, where one row per thread fits,
+ *                            (0, built-in) or, where one row per thread fits
+ *                            and HBEM_TUNE_LU_PANEL does not choose the whole
+ *                            block launch,
  *                            in registers (1: 64 columns up to 384 rows, 32
  *                            up to 768, 16 up to 1024); the factors are the
  *                            same bits
