@@ -1492,7 +1492,13 @@ int launch_regular(Session &s, int n_freq, const float *k_re, const float *k_im,
                    float *a_im, long long lda, long long a_stride, float *b_re, float *b_im, long long b_stride,
                    cudaStream_t st, int n_src, long long q_src_stride, long long b_src_stride) {
     if (n_src < 1 || n_src > kMaxSources) return fail(HBEM_ERR_ARG, "assembly: 1 .. 8 sources per pass");
+    // The ordered kernel's 64-triangle trial tiles can need more shared memory
+    // than there is where few triangles share vertices; the unordered kernel's
+    // 8-triangle chunks never do (at most 4 planes of 24 x 97 dofs, 149 KB)
+    const bool ordered = tuning(HBEM_TUNE_ASM_PAIRS) == 1 && n_src == 1;
     const size_t smem = (size_t)kAsmFreqs * (s.max_rows * (s.max_cols | 1) + s.max_rows) * sizeof(float2);
+    if (ordered && smem > 180 * 1024)
+        return fail(HBEM_ERR_ARG, "assembly tile needs too much shared memory (mesh ordering too scattered)");
     static bool consts_ready[64] = {false};
     if (s.device >= 0 && s.device < 64 && !consts_ready[s.device]) {
         const double QX[6] = {0.4459484909159651, 0.0915762135097710, 0.1081030181680700,
@@ -1516,8 +1522,6 @@ int launch_regular(Session &s, int n_freq, const float *k_re, const float *k_im,
         HBEM_CUDA(cudaMemcpyToSymbol(c_wa2, wa2, sizeof(wa2)));
         consts_ready[s.device] = true;
     }
-    if (smem > 180 * 1024)
-        return fail(HBEM_ERR_ARG, "assembly tile needs too much shared memory (mesh ordering too scattered)");
     for (int f0 = 0; f0 < n_freq; f0 += kMaxFreqPerLaunch) {
         const int nf = std::min(kMaxFreqPerLaunch, n_freq - f0);
         AsmArgs a{};
@@ -1539,7 +1543,7 @@ int launch_regular(Session &s, int n_freq, const float *k_re, const float *k_im,
         if (!a.b_re) a.q_re = a.q_im = nullptr;
         a.nf = nf;
         cudaError_t e;
-        if (tuning(HBEM_TUNE_ASM_PAIRS) != 1 || n_src > 1) {
+        if (!ordered) {
             a.chunk_slot = s.d_chunk_slot; a.chunk_off = s.d_chunk_off; a.chunk_cols = s.d_chunk_cols;
             a.gather = s.d_gather;
             a.plane = s.max_chunk_cols * (s.max_rows | 1);

@@ -3,6 +3,8 @@ from __future__ import annotations
 
 import json
 
+import pytest
+
 from hornlab_metal_bem_b200.batch import CANDIDATES, Autotuner, lpt_slots, size_bucket
 
 
@@ -56,6 +58,18 @@ def test_autotuner_picks_fastest_per_bucket_and_caches(tmp_path):
     t3.tune(cases)
     assert len(calls) == 2 * len(CANDIDATES)
     assert set(json.loads(cache.read_text())) == {"gpu-x|1", "gpu-y|1"}
+
+
+def test_autotuner_leaves_out_variants_that_refuse_a_mesh(tmp_path):
+    def timer(case, variant):
+        if variant["pairs"] == 1 or case.n < 0:
+            raise RuntimeError("refused")
+        return 1.0 if variant["panel"] == 16 else 2.0
+
+    t = Autotuner(timer, "gpu-x|1", tmp_path / "tune.json")
+    assert t.tune([_Case(500)])["n<=768"]["panel"] == 16
+    with pytest.raises(RuntimeError):   # the built-in variant has to run
+        t.tune([_Case(-1)], force=True)
 
 
 def test_matrix_pitch_and_solve_names():

@@ -46,8 +46,18 @@ def _apart(n):
     return mesh_from_arrays(v, np.arange(3 * n, dtype=np.int32).reshape(n, 3), np.ones(n, np.int32))
 
 
+def _scattered():
+    """70 triangles without a common vertex: more dofs in a 64-triangle tile than the ordered kernel can stage, which
+    is no limit of the unordered one.  k r reaches 26 here, 1.6e-6 of the tolerance."""
+    rng = np.random.default_rng(4)
+    c = np.stack(np.meshgrid(np.arange(4), np.arange(4), np.arange(5), indexing="ij"), -1).reshape(-1, 3)[:70] * 0.1
+    v = (c[:, None] + 0.02 * rng.standard_normal((70, 3, 3))).reshape(-1, 3)
+    return mesh_from_arrays(v, np.arange(210, dtype=np.int32).reshape(70, 3), np.ones(70, np.int32))
+
+
 MESHES = {"one_tile": (lambda: G.icosphere(0, 0.1), None, 0), "ragged": (lambda: G.icosphere(1, 0.1), None, 0),
           "fan": (lambda: _fan(37), None, 0), "apart": (lambda: _apart(38), None, 0),
+          "scattered": (_scattered, None, 0),
           "quarter": (lambda: G.horn(G.HornSpec(edge=0.02), quarter=True), "yz+xz", 3),
           "half": (lambda: G.horn(G.HornSpec(edge=0.03), quarter=False, half=True), "yz", 1)}
 
