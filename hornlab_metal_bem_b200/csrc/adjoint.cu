@@ -304,9 +304,9 @@ __global__ void __launch_bounds__(kBwdThreads, 2) k_asm_bwd(const __grid_constan
         const int t = s0 + i;
         int driven = 0;
         for (int f = 0; f < 2 * np; ++f) {
-            const bool in = t < T && f < nf && a.q_re && a.q_im;
-            const float qr = in ? a.q_re[(size_t)f * a.q_stride + t] : 0.f;
-            const float qi = in ? a.q_im[(size_t)f * a.q_stride + t] : 0.f;
+            const bool in = t < T && f < nf;
+            const float qr = in && a.q_re ? a.q_re[(size_t)f * a.q_stride + t] : 0.f;
+            const float qi = in && a.q_im ? a.q_im[(size_t)f * a.q_stride + t] : 0.f;
             float *to = sQ + 4 * ((f >> 1) * kBwdTrial + i) + (f & 1);
             to[0] = qr;
             to[2] = qi;

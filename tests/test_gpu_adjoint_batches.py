@@ -46,3 +46,31 @@ def test_assembly_gradient_sums_over_frequencies(freqs, level):
         whole = grad(0, freqs)
         single = sum(grad(f, f + 1) for f in range(freqs))
     assert np.linalg.norm(whole - single) <= 2e-5 * np.linalg.norm(single)
+
+
+@pytest.mark.parametrize("missing", ["real", "imaginary"])
+def test_neumann_data_of_one_part_only(missing):
+    """A NULL part of the Neumann data is a part of zeros, for regular and touching pairs alike."""
+    mesh = G.icosphere(1, 0.1)
+    p1, dp0 = make_pure_function_spaces(mesh.grid)
+    b = build_geometry_buffers(mesh.grid, mesh.physical_tags, p1, dp0)
+    n, T, V = b.p1_dof_count, b.n_triangles, np.asarray(b.vertices_3xn_f32).shape[1]
+    rng = np.random.default_rng(7)
+    k = np.array([5.0, 30.0], np.float32)
+    dev = torch.device("cuda")
+    lam, p = (torch.tensor(rng.standard_normal((2, 2, n)), dtype=torch.float32, device=dev) for _ in range(2))
+    q = torch.tensor(rng.standard_normal((2, T)), dtype=torch.float32, device=dev)
+    with NativeSession(b, check_open_edges=False) as s:
+        def grad(q_re, q_im):
+            out = torch.zeros((3, V), dtype=torch.float64, device=dev)
+            check(s.lib.hbem_assemble_backward(
+                s.handle, 2, _np_ptr(k), None, _t_ptr(lam[0]), _t_ptr(lam[1]), n, _t_ptr(p[0]), _t_ptr(p[1]), n,
+                _t_ptr(q_re), _t_ptr(q_im), T, _t_ptr(out), _stream_ptr()), "hbem_assemble_backward")
+            torch.cuda.synchronize()
+            return out.cpu().numpy()
+
+        zero = torch.zeros_like(q)
+        one, both = (grad(None, q), grad(zero, q)) if missing == "real" else (grad(q, None), grad(q, zero))
+        without = grad(None, None)
+    assert np.linalg.norm(both - without) > 0.01 * np.linalg.norm(both)   # the Neumann data matter
+    assert np.linalg.norm(one - both) <= 2e-5 * np.linalg.norm(both)
