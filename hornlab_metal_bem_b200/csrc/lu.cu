@@ -830,12 +830,14 @@ __global__ void __launch_bounds__(kBlkMaxRows) k_panel_block(float *a_re, float 
             wk = __reduce_max_sync(0xffffffffu, key);
             wp = __reduce_min_sync(0xffffffffu, active && key == wk ? pos : kNoRow);
         };
-        // the best of `count` <= 16 candidates (key, position, local row): its index
+        // the best of `count` <= 16 candidates (key, position, local row): its index, below `count` also where
+        // a wait that ran out has left them unwritten
         auto best_of = [&](const uint4 *cand, int count) -> int {
             const uint2 c = lane < count ? *reinterpret_cast<const uint2 *>(cand + lane)
                                          : make_uint2(0u, (unsigned)kNoRow);
             const unsigned bk = __reduce_max_sync(0xffffffffu, c.x);
-            return (int)(__reduce_min_sync(0xffffffffu, c.x == bk ? c.y << 4 | (lane & 15) : 0xffffffffu) & 15u);
+            const unsigned w = __reduce_min_sync(0xffffffffu, c.x == bk ? c.y << 4 | (lane & 15) : 0xffffffffu);
+            return min((int)(w & 15u), count - 1);
         };
         warp_best(q0);
 #pragma unroll 1
