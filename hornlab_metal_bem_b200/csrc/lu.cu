@@ -798,6 +798,9 @@ __global__ void __launch_bounds__(kBlkMaxRows) k_panel_block(float *a_re, float 
         }
     }
     for (int e = tid; e < kBlkW * kBlkW; e += blockDim.x) S.l[e / kBlkW][e % kBlkW] = make_float2(0.f, 0.f);
+    // (what a wait that runs out finds in place of a CTA's candidate)
+    if (CLUSTER && tid < 2 * kBlkMaxCta)
+        S.gcand[tid / kBlkMaxCta][tid % kBlkMaxCta] = make_uint4(0u, (unsigned)kNoRow, 0u, 0u);
     if (CLUSTER && tid == 0) {
         for (int i = 0; i < 2; ++i)
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&S.bar[i])));
@@ -830,14 +833,13 @@ __global__ void __launch_bounds__(kBlkMaxRows) k_panel_block(float *a_re, float 
             wk = __reduce_max_sync(0xffffffffu, key);
             wp = __reduce_min_sync(0xffffffffu, active && key == wk ? pos : kNoRow);
         };
-        // the best of `count` <= 16 candidates (key, position, local row): its index, below `count` also where
-        // a wait that ran out has left them unwritten
+        // the best of `count` <= 16 candidates (key, position, local row): its index, below `count` as no
+        // position passes kNoRow
         auto best_of = [&](const uint4 *cand, int count) -> int {
             const uint2 c = lane < count ? *reinterpret_cast<const uint2 *>(cand + lane)
                                          : make_uint2(0u, (unsigned)kNoRow);
             const unsigned bk = __reduce_max_sync(0xffffffffu, c.x);
-            const unsigned w = __reduce_min_sync(0xffffffffu, c.x == bk ? c.y << 4 | (lane & 15) : 0xffffffffu);
-            return min((int)(w & 15u), count - 1);
+            return (int)(__reduce_min_sync(0xffffffffu, c.x == bk ? c.y << 4 | (lane & 15) : 0xffffffffu) & 15u);
         };
         warp_best(q0);
 #pragma unroll 1
