@@ -2260,6 +2260,20 @@ __global__ void k_rc_init(int n, float *x_re, float *x_im, long long stride, RcS
     }
 }
 
+// w = x for the matrices in states lo .. hi, marked in active[] (w is then
+// solved in place by a forced scheme)
+__global__ void k_rc_copy(int n, const float *x_re, const float *x_im, float *w_re, float *w_im, long long stride,
+                          const RcState *state, int lo, int hi, int *active) {
+    const int mat = blockIdx.y;
+    const bool want = state[mat].st >= lo && state[mat].st <= hi;
+    if (blockIdx.x == 0 && threadIdx.x == 0) active[mat] = want ? 1 : 0;
+    if (!want) return;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        w_re[(size_t)mat * stride + i] = x_re[(size_t)mat * stride + i];
+        w_im[(size_t)mat * stride + i] = x_im[(size_t)mat * stride + i];
+    }
+}
+
 __device__ void block_sum_max(double &sum, float &mx, int &imx) {
     __shared__ double s_sum[32];
     __shared__ float s_mx[32];
@@ -3397,8 +3411,14 @@ int lu_rcond(int n, int batch, const float *lu_re, const float *lu_im, long long
     constexpr int kSolves = 1 + 2 * (kItMax + 1);
     const long long stride = n;
     const size_t vec = (sizeof(float) * 2 * (size_t)batch * n + 255) & ~(size_t)255;
-    const size_t box = (both_scratch_bytes(batch, n) + 255) & ~(size_t)255;
-    const int boxes = box * kSolves <= (32u << 20) ? kSolves : 1;
+    // a scheme forced by HBEM_TUNE_LU_SOLVE takes the solves too (x copied to w
+    // and solved in place); the box is then the wavefront's scratch and the
+    // matrices' active flags
+    const bool forced = tuning(HBEM_TUNE_LU_SOLVE) != 0;
+    const size_t wave = (wave_scratch_bytes(batch, n) + 255) & ~(size_t)255;
+    const size_t box = forced ? wave + ((sizeof(int) * batch + 255) & ~(size_t)255)
+                              : (both_scratch_bytes(batch, n) + 255) & ~(size_t)255;
+    const int boxes = !forced && box * kSolves <= (32u << 20) ? kSolves : 1;
     const size_t states = (sizeof(RcState) * batch + 255) & ~(size_t)255;
     unsigned char *mem = nullptr;
     HBEM_CUDA(cudaMallocAsync((void **)&mem, 2 * vec + states + box * boxes, st));
@@ -3416,6 +3436,14 @@ int lu_rcond(int n, int batch, const float *lu_re, const float *lu_im, long long
     };
     // op(LU) w = x for the matrices in states lo .. hi
     auto solve = [&](int trans, int lo, int hi) {
+        if (forced) {
+            int *active = reinterpret_cast<int *>(mbox + wave);
+            k_rc_copy<<<gv, 256, 0, st>>>(n, xr, xi, wr, wi, stride, state, lo, hi, active);
+            if (launched("k_rc_copy"))
+                rc = lu_solve_ex(n, 1, batch, lu_re, lu_im, lda, a_stride, nullptr, n, wr, wi, 1, stride, trans, active,
+                                 mbox, st);
+            return rc == HBEM_OK;
+        }
         unsigned char *b = mbox + (boxes > 1 ? box * solves : 0);
         if (boxes == 1 || solves == 0) {
             const cudaError_t e = cudaMemsetAsync(b, 0xff, box * boxes, st);

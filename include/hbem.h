@@ -108,9 +108,10 @@ long long hbem_launch_count(void);
  *   HBEM_TUNE_LU_SOLVE:      triangular solves (1: one CTA per right-hand
  *                            side, 2: blocked multi-CTA steps, 3: wavefront,
  *                            one CTA per 32-row block; 0: one CTA per
- *                            right-hand side for n <= 128, else wavefront,
- *                            refinement and condition estimate with both
- *                            triangular phases in one launch up to n = 25600)
+ *                            right-hand side for n <= 128, else wavefront;
+ *                            refinement with n > 128, and the condition
+ *                            estimate with any n, run both triangular phases
+ *                            in one launch)
  *   HBEM_TUNE_ASM_PAIRS:     regular assembly (0: unordered pairs, both
  *                            orders and two wavenumbers from one kernel
  *                            evaluation; 1: ordered pairs, two wavenumbers)

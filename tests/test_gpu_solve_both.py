@@ -58,3 +58,39 @@ def test_refined_solution_and_condition_estimate(n, batch):
         lu, _, _ = lapack.cgetrf(A[m])
         want, _ = lapack.cgecon(lu, np.abs(A[m]).sum(0).max().astype(np.float32), norm="1")
         assert abs(float(rcond[m]) - want) <= 1e-2 * want
+
+
+HBEM_TUNE_LU_SOLVE = 2
+
+
+@pytest.mark.parametrize("mode", [1, 2, 3])
+def test_forced_solve_schemes_take_the_condition_estimate(mode):
+    """HBEM_TUNE_LU_SOLVE: every solve of the estimate is the forced scheme's (a copy and at least one launch of its
+    own, 13 times), not the built-in one; the same 1 % to cgecon."""
+    lib = load_library()
+    n, batch = 161, 2
+    rng = np.random.default_rng(3)
+    A = (rng.standard_normal((batch, n, n)) + 1j * rng.standard_normal((batch, n, n))).astype(np.complex64)
+    Ar, Ai = _parts(A)
+    piv = torch.empty((batch, n), dtype=torch.int32, device="cuda")
+    info = torch.empty(batch, dtype=torch.int32, device="cuda")
+    anorm = torch.tensor(np.abs(A).sum(1).max(1), device="cuda")
+    rcond = torch.empty(batch, dtype=torch.float64, device="cuda")
+    st = _stream_ptr()
+    check(lib.hbem_lu_factor(n, batch, _t_ptr(Ar), _t_ptr(Ai), n, n * n, _t_ptr(piv), n, _t_ptr(info), HBEM_PREC_TF32X3,
+                             st), "hbem_lu_factor")
+    launches = {}
+    try:
+        for m in (0, mode):
+            check(lib.hbem_set_tuning(HBEM_TUNE_LU_SOLVE, m), "hbem_set_tuning")
+            before = int(lib.hbem_launch_count())
+            check(lib.hbem_lu_rcond(n, batch, _t_ptr(Ar), _t_ptr(Ai), n, n * n, _t_ptr(anorm), _t_ptr(rcond), st),
+                  "hbem_lu_rcond")
+            launches[m] = int(lib.hbem_launch_count()) - before
+            for i in range(batch):
+                lu, _, _ = lapack.cgetrf(A[i])
+                want, _ = lapack.cgecon(lu, np.abs(A[i]).sum(0).max().astype(np.float32), norm="1")
+                assert abs(float(rcond[i]) - want) <= 1e-2 * want
+    finally:
+        lib.hbem_set_tuning(HBEM_TUNE_LU_SOLVE, 0)
+    assert launches[mode] >= launches[0] + 13
