@@ -3027,7 +3027,8 @@ int lu_factor(int n, int batch, float *a_re, float *a_im, long long lda, long lo
     // 64-column panels and their roundings: without refinement another order
     // of the same sums moves the solution of an ill-conditioned system as far
     // as its error (a shape gradient at n = 2082 by 2e-4).
-    const bool block_panels = precision != HBEM_PREC_PLAIN && tuning(HBEM_TUNE_LU_PANEL) == 0;
+    const bool block_panels = precision != HBEM_PREC_PLAIN && tuning(HBEM_TUNE_LU_PANEL) == 0 &&
+                              tuning(HBEM_TUNE_LU_PANEL_KERNEL) == 0;
     // net row moves of the blocks k_panel_block factors
     BlkMoves *moves = nullptr, *block_moves = nullptr;   // all blocks', and the current block's (NULL: from piv)
     if (block_panels) {

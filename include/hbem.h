@@ -102,7 +102,8 @@ long long hbem_launch_count(void);
  *                            it, else 16 where one CTA holds it, else 32 in
  *                            a cluster; 64: as 0, but the whole block also
  *                            in an 8-CTA cluster where that holds it).  With
- *                            0, HBEM_PREC_TF32X3 and HBEM_PREC_MIXED factor
+ *                            0 here and in HBEM_TUNE_LU_PANEL_KERNEL,
+ *                            HBEM_PREC_TF32X3 and HBEM_PREC_MIXED factor
  *                            whole 64-column blocks of up to 6144 rows in one
  *                            launch instead
  *   HBEM_TUNE_LU_SOLVE:      triangular solves (1: one CTA per right-hand
@@ -142,9 +143,7 @@ long long hbem_launch_count(void);
  *                            built-in 128 for n > 16000, else 64); the FP32
  *                            LU's TF32x3 bulk takes K = 64 with any value
  *   HBEM_TUNE_LU_PANEL_KERNEL: sub-panels with their rows in shared memory
- *                            (0, built-in) or, where one row per thread fits
- *                            and HBEM_TUNE_LU_PANEL does not choose the whole
- *                            block launch,
+ *                            (0, built-in) or, where one row per thread fits,
  *                            in registers (1: 64 columns up to 384 rows, 32
  *                            up to 768, 16 up to 1024); the factors are the
  *                            same bits

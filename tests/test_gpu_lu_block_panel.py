@@ -16,10 +16,10 @@ if not torch.cuda.is_available():  # pragma: no cover - CPU containers
 
 from hornlab_metal_bem_b200.native import HBEM_PREC_TF32X3, _stream_ptr, _t_ptr, check, load_library  # noqa: E402
 
-HBEM_TUNE_LU_UPDATE = 8
+HBEM_TUNE_LU_PANEL, HBEM_TUNE_LU_UPDATE, HBEM_TUNE_LU_PANEL_KERNEL = 1, 8, 10
 
 
-def _factor(A, ld):
+def _factor(A, ld, panel=0, kernel=0):
     lib = load_library()
     F, n = A.shape[:2]
     planes = np.zeros((2, F, n, ld), np.float32)
@@ -29,10 +29,13 @@ def _factor(A, ld):
     info = torch.empty(F, dtype=torch.int32, device="cuda")
     check(lib.hbem_set_tuning(HBEM_TUNE_LU_UPDATE, 1), "hbem_set_tuning")   # exact FP32 products in the bulk
     try:
+        check(lib.hbem_set_tuning(HBEM_TUNE_LU_PANEL, panel), "hbem_set_tuning")
+        check(lib.hbem_set_tuning(HBEM_TUNE_LU_PANEL_KERNEL, kernel), "hbem_set_tuning")
         check(lib.hbem_lu_factor(n, F, _t_ptr(re), _t_ptr(im), ld, n * ld, _t_ptr(piv), n, _t_ptr(info), HBEM_PREC_TF32X3,
                                  _stream_ptr()), "hbem_lu_factor")
     finally:
-        lib.hbem_set_tuning(HBEM_TUNE_LU_UPDATE, 0)
+        for knob in (HBEM_TUNE_LU_UPDATE, HBEM_TUNE_LU_PANEL, HBEM_TUNE_LU_PANEL_KERNEL):
+            lib.hbem_set_tuning(knob, 0)
     check(lib.hbem_solve_status(_stream_ptr()), "hbem_solve_status")
     LU = (re.double() + 1j * im.double())[:, :, :n].cpu().numpy()
     return LU, piv.cpu().numpy(), info.cpu().numpy()
@@ -86,3 +89,12 @@ def test_block_panel_is_bitwise_stable_under_concurrent_work():
         busy = _factor(A, 1044)
         assert all(np.array_equal(a, b) for a, b in zip(quiet, busy))
     torch.cuda.synchronize()
+
+
+def test_register_sub_panels_stay_selectable_for_refined_factors():
+    """HBEM_TUNE_LU_PANEL_KERNEL = 1 takes the register sub-panels, whose factors are the shared-memory ones' bits
+    (HBEM_TUNE_LU_PANEL = 64), in place of the whole-block launch."""
+    rng = np.random.default_rng(6)
+    A = (rng.standard_normal((2, 300, 300)) + 1j * rng.standard_normal((2, 300, 300))).astype(np.complex64)
+    registers, shared = _factor(A, 300, kernel=1), _factor(A, 300, panel=64)
+    assert all(np.array_equal(a, b) for a, b in zip(registers, shared))
