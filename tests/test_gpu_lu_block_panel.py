@@ -53,15 +53,18 @@ def _permuted(A, piv):
 def test_block_panel_factors(n, pad):
     rng = np.random.default_rng(n)
     A = (rng.standard_normal((2, n, n)) + 1j * rng.standard_normal((2, n, n))).astype(np.complex64)
-    A[1, :, n // 2] *= 1e-20   # a column whose pivots' squares leave the FP32 range
+    # columns whose pivots' squares leave the FP32 range, or lie at the ends of the unscaled reciprocal's
+    for col, scale in zip([n // 2, n // 3, n - 1, 0], [1e-20, 1e16, 1e-16, 1e18]):
+        A[1, :, col] *= np.float32(scale)
     LU, piv, info = _factor(A, n + pad)
     assert not info.any()
     for m in range(2):
         L, U = np.tril(LU[m], -1) + np.eye(n), np.triu(LU[m])
         assert np.abs(np.tril(LU[m], -1)).max(initial=0.0) <= np.sqrt(2.0) * (1 + 1e-5)
-        if m == 0:
-            ref = _permuted(A[m].astype(np.complex128), piv[m])
-            assert np.linalg.norm(L @ U - ref) <= 1e-5 * np.linalg.norm(ref)
+        # each column over its own norm, so that the scaled ones count as the others
+        ref = _permuted(A[m].astype(np.complex128), piv[m])
+        size = np.linalg.norm(ref, axis=0)
+        assert np.linalg.norm((L @ U - ref) / size) <= 1e-5 * np.sqrt(n)
 
 
 @pytest.mark.parametrize("n,col", [(40, 0), (200, 17), (500, 70)])
@@ -98,3 +101,20 @@ def test_register_sub_panels_stay_selectable_for_refined_factors():
     A = (rng.standard_normal((2, 300, 300)) + 1j * rng.standard_normal((2, 300, 300))).astype(np.complex64)
     registers, shared = _factor(A, 300, kernel=1), _factor(A, 300, panel=64)
     assert all(np.array_equal(a, b) for a, b in zip(registers, shared))
+
+
+def test_multipliers_use_a_correctly_rounded_reciprocal():
+    """Column 0: multipliers x * conj(d) (1 / |d|^2) with every operation rounded once to FP32 (longdouble holds the
+    exact products and, but for a tie's last bit, the sums), bit for bit over 400 pivots."""
+    rng = np.random.default_rng(8)
+    A = (rng.standard_normal((400, 20, 20)) + 1j * rng.standard_normal((400, 20, 20))).astype(np.complex64)
+    LU, piv, _ = _factor(A, 20)
+    f32, wide = np.float32, np.longdouble
+    fma = lambda a, b, c: (wide(a) * wide(b) + wide(c)).astype(f32)  # noqa: E731
+    for m in range(400):
+        x = _permuted(A[m], piv[m])[:, 0]
+        xr, xi, dr, di = x.real[1:], x.imag[1:], x.real[:1], x.imag[:1]
+        den = f32(1.0) / fma(dr, dr, di * di)
+        ir, ii = dr * den, -di * den
+        assert np.array_equal(LU[m, 1:, 0].real.astype(f32), fma(xr, ir, -(xi * ii)))
+        assert np.array_equal(LU[m, 1:, 0].imag.astype(f32), fma(xr, ii, xi * ir))
