@@ -72,6 +72,16 @@ def test_autotuner_leaves_out_variants_that_refuse_a_mesh(tmp_path):
         t.tune([_Case(-1)], force=True)
 
 
+def test_picks_saved_by_an_earlier_library_are_timed_again(tmp_path):
+    """Version 100 timed other kernels behind the same knobs."""
+    from hornlab_metal_bem_b200.native import load_library
+
+    cache = tmp_path / "tune.json"
+    Autotuner(lambda case, v: 1.0 if v["panel"] == 16 else 2.0, "gpu-x|100", cache).tune([_Case(500)])
+    now = Autotuner(lambda case, v: 1.0 if v["panel"] == 0 else 2.0, f"gpu-x|{load_library().hbem_version()}", cache)
+    assert now.tune([_Case(500)])["n<=768"]["panel"] == 0
+
+
 def test_matrix_pitch_and_solve_names():
     """The sweep paths' dense row pitch is n rounded up to 4 floats (16-byte rows), and a refined plain
     solve is reported as the FP32 LU with the TF32x3 tensor-core bulk."""
