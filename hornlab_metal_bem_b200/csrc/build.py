@@ -23,7 +23,7 @@ REPO = PKG.parent
 OUT = PKG / "libhbem.so"
 BUILD = REPO / "_build" / "hbem"
 SOURCES = ["session.cu", "assemble.cu", "field.cu", "lu.cu", "gemm.cu", "sweep.cu", "aperture.cu", "adjoint.cu", "fp64.cu", "near.cu"]
-HEADERS = ["hbem_internal.h"]
+HEADERS = ["hbem_internal.h", "triangle_order.h"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", "-O3",
          "--expt-relaxed-constexpr", "-I", str(REPO / "include")]
