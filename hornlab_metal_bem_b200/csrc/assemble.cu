@@ -1030,7 +1030,8 @@ cudaError_t launch_pairs(AsmArgs a, int tiles_x, int tiles_y, cudaStream_t st, i
         a.f_base = 0;
         const int groups = a.nf > 1 ? (a.nf + 1) / 2 : 1;
         a.rhs_block = kRhsTrials;
-        while (a.rhs_block > 32 && tiles_y * ((a.T + a.rhs_block - 1) / a.rhs_block) * groups < 6 * 148)
+        while (a.rhs_block > 32 &&
+               (long long)tiles_y * ((a.T + a.rhs_block - 1) / a.rhs_block) * groups < 6 * sm_count())
             a.rhs_block /= 2;
         const int tx = (a.T + a.rhs_block - 1) / a.rhs_block;
         const dim3 g2(tx, tiles_y, (a.nf + 1) / 2), g1(tx, tiles_y, a.nf);

@@ -233,7 +233,7 @@ int launch_field(Session &s, int n_freq, const float *k_re, const float *p_re, c
             a.k[f] = k_re[f0 + f];
             a.kt[f] = (double)k_re[f0 + f] / (2.0 * 3.14159265358979323846);
         }
-        if ((n_obs + 7) / 8 * nf < 2 * 148) launch_field_t<2>(s.sym, a, nf, st);
+        if ((n_obs + 7LL) / 8 * nf < 2 * sm_count()) launch_field_t<2>(s.sym, a, nf, st);
         else launch_field_t<8>(s.sym, a, nf, st);
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return cuda_fail(e, "k_field launch");

@@ -144,7 +144,7 @@ int launch_trailing_simt(int n, int batch, int k0, int kw, int start, int col_st
     // 64 columns at n = 1043, one matrix: 16 CTAs of 64; the same sums in the
     // same order): factorisation of 642 x 8 1266 -> 1228 us, 1043 x 1 2122 -> 2098
     const long long tiles = (long long)((w + 63) / 64) * ((m + 63) / 64) * batch;
-    if (tiles < 148) {
+    if (tiles < sm_count()) {
         const dim3 grid((w + 63) / 64, (m + 31) / 32, batch);
         k_trailing_simt<32><<<grid, 256, 0, st>>>(a_re, a_im, lda, a_stride, n, k0, kw, start, col_start, col_end);
     } else {
@@ -933,11 +933,8 @@ int launch_trailing_tc_t(TcWorkspace *w, int n, int batch, int k0, int start, in
                                                 tiles_n * Cfg::N, static_cast<T *>(w->B2));
         HBEM_LAUNCH_CHECK("k_pack_b");
     }
-    int n_sm = 0;
+    const int n_sm = sm_count();
     {
-        int dev = 0;
-        HBEM_CUDA(cudaGetDevice(&dev));
-        HBEM_CUDA(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev));
         const int rc = func_opt_in((const void *)k_trailing_tc<TF32, KC>, (int)Cfg::Smem);
         if (rc != HBEM_OK) return rc;
     }

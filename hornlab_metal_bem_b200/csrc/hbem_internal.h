@@ -20,6 +20,7 @@ int tuning(int key);   // HBEM_TUNE_* value, 0 = built-in choice
 void keep_pool_memory();   // cache freed stream-ordered allocations of the current device
 // raise a kernel's dynamic shared-memory limit once per device (thread-safe)
 int func_opt_in(const void *func, int smem_bytes, bool nonportable_cluster = false);
+int sm_count();
 
 #define HBEM_CUDA(call)                                        \
     do {                                                       \

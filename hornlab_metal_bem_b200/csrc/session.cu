@@ -56,6 +56,17 @@ int func_opt_in(const void *func, int smem_bytes, bool nonportable_cluster) {
     return HBEM_OK;
 }
 
+// SMs of the current device (a partition may have fewer than the part)
+int sm_count() {
+    static std::atomic<int> cached[64];
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
+    if ((n = cached[dev].load()) > 0) return n;
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) return 148;
+    cached[dev].store(n);
+    return n;
+}
+
 // Stream-ordered allocations (workspaces of the LU, refinement, condition
 // estimate) come from the device's default memory pool; by default that pool
 // hands freed memory back to the driver at every synchronisation, so the
