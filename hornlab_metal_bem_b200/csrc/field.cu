@@ -8,8 +8,14 @@
 // to the 6 quadrature points once per triangle, and accumulate the tile's
 // observation sums in registers before a block reduction (the same order of
 // sums for either tile).  111 points at one frequency on the quarter horn of
-// 1950 triangles are 14 CTAs of 8 points (373 us) or 56 of 2 (60 us); from 296
-// CTAs of 8 on, two per SM, the larger tile shares more of the interpolation.
+// 1950 triangles are 14 CTAs of 8 points (373 us) or 56 of 2 (60 us).  The
+// larger tile shares the interpolation of more points but needs two CTAs an SM
+// to hide its latency: below that (296 CTAs of 8), 2 points a CTA.  With four
+// images its one or two CTAs an SM take the same 0.36 ms (1986 triangles),
+// which 2 points a CTA reach between seven and eight CTAs an SM (2072 points
+// 0.339 ms, 2200 0.360, 2360 0.384): there the line is at seven.  With one or
+// two images 2200 points take 0.31-0.34 ms in CTAs of 8, 0.26-0.29 in CTAs of 2
+// (2968 and 5886 triangles).
 // Tag averages (main.swift:807-841) use FP64 block sums.
 //
 // Phase accuracy: at 2 m and 20 kHz, k r is ~730 rad, so an FP32 distance
@@ -233,7 +239,8 @@ int launch_field(Session &s, int n_freq, const float *k_re, const float *p_re, c
             a.k[f] = k_re[f0 + f];
             a.kt[f] = (double)k_re[f0 + f] / (2.0 * 3.14159265358979323846);
         }
-        if ((n_obs + 7LL) / 8 * nf < 2 * sm_count()) launch_field_t<2>(s.sym, a, nf, st);
+        const bool small = s.sym == 3 ? (n_obs + 1LL) / 2 * nf <= 7 * sm_count() : (n_obs + 7LL) / 8 * nf < 2 * sm_count();
+        if (small) launch_field_t<2>(s.sym, a, nf, st);
         else launch_field_t<8>(s.sym, a, nf, st);
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return cuda_fail(e, "k_field launch");
