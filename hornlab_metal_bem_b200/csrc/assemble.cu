@@ -191,7 +191,7 @@ __device__ __forceinline__ void sample2_w(float dx, float dy, float dz, float nx
 
 template <int SYM, int NF, bool CK, bool NEED_G>
 __device__ __forceinline__ void pair_block(const float4 *__restrict__ tq, const float4 *__restrict__ sp, float nx,
-                                           float ny, float nz, bool self, const float (&k)[NF],
+                                           float ny, float nz, const float (&k)[NF],
                                            const float (&ki)[NF], float (&are)[NF][9],
                                            float (&aim)[NF][9], float (&sre)[NF][3], float (&sim)[NF][3]) {
 #pragma unroll
@@ -220,8 +220,7 @@ __device__ __forceinline__ void pair_block(const float4 *__restrict__ tq, const 
             float dre[NF], dim[NF], gre[NF], gim[NF];
 #pragma unroll
             for (int f = 0; f < NF; ++f) dre[f] = dim[f] = gre[f] = gim[f] = 0.f;
-            if (!(self && a == b))
-                sample_nf<NF, CK, NEED_G>(y.x - x.x, y.y - x.y, y.z - x.z, nx, ny, nz, k, ki, dre, dim, gre, gim);
+            sample_nf<NF, CK, NEED_G>(y.x - x.x, y.y - x.y, y.z - x.z, nx, ny, nz, k, ki, dre, dim, gre, gim);
             if (SYM == 1 || SYM == 3)
                 sample_nf<NF, CK, NEED_G>(-y.x - x.x, y.y - x.y, y.z - x.z, -nx, ny, nz, k, ki, dre, dim, gre, gim);
             if (SYM == 2 || SYM == 3)
@@ -266,6 +265,11 @@ __device__ __forceinline__ void pair_block(const float4 *__restrict__ tq, const 
 
 // blockIdx.z selects a group of NF consecutive frequencies; a missing last
 // member (odd count) is computed on a repeated wavenumber and not flushed.
+// Lane t holds its test triangle's vertices turned by t mod 3: neighbours in the
+// triangle order share a vertex in the same place, where the shared atomics of
+// 32 lanes would meet on one address (1986 triangles, 4 images, 40
+// wavenumbers 25.2 ms unturned, 20.3 turned).  The coincident point of a
+// triangle with itself drops out in sample_nf (r^2 = 0).
 template <int SYM, bool CK, int MINB>
 __global__ void __launch_bounds__(kAsmThreads, MINB) k_regular(const __grid_constant__ AsmArgs p) {
     constexpr int NF = kAsmFreqs;
@@ -294,8 +298,11 @@ __global__ void __launch_bounds__(kAsmThreads, MINB) k_regular(const __grid_cons
     for (int i = tid; i < NF * plane; i += kAsmThreads) s_acc[i] = make_float2(0.f, 0.f);
     for (int i = tid; i < ntrial * 6; i += kAsmThreads) s_qp[i] = p.qp[(size_t)tbase * 6 + i];
     for (int i = tid; i < ntest * 6; i += kAsmThreads) {
-        const int t = i / 6, a = i - 6 * t;
-        s_tq[a * kTestTile + t] = p.qp[(size_t)(test0 + t) * 6 + a];
+        // rule point a belongs to vertex l, whose place is `to`; the rule's orbits are points 0 2 3 and 1 4 5
+        const int t = i / 6, a = i - 6 * t, l = a < 2 ? 0 : (a == 2 || a == 4 ? 1 : 2);
+        const int to = (l + 3 - t % 3) % 3;
+        const int point = a == 1 || a > 3 ? (to == 0 ? 1 : to + 3) : (to == 0 ? 0 : to + 1);
+        s_tq[point * kTestTile + t] = p.qp[(size_t)(test0 + t) * 6 + a];
     }
     for (int i = tid; i < ntrial; i += kAsmThreads) {
         s_nrm[i] = p.nrm[tbase + i];
@@ -331,17 +338,18 @@ __global__ void __launch_bounds__(kAsmThreads, MINB) k_regular(const __grid_cons
     if (lane < ntest) {
         const float tjac = p.nrm[test].w;
         const uchar4 rs = p.test_slot[test];
-        const int rslot[3] = {rs.x, rs.y, rs.z};
+        const int rot = lane % 3;   // place i of this lane holds vertex (i + rot) % 3
+        const int rslot[3] = {rot == 0 ? rs.x : (rot == 1 ? rs.y : rs.z), rot == 0 ? rs.y : (rot == 1 ? rs.z : rs.x),
+                              rot == 0 ? rs.z : (rot == 1 ? rs.x : rs.y)};
         const float4 *tq = &s_tq[lane];
         for (int jj = warp; jj < ntrial; jj += kAsmThreads / 32) {
             const float4 nj = s_nrm[jj];
             const bool self = (tbase + jj) == test;
             float are[NF][9], aim[NF][9], sre[NF][3], sim[NF][3];
             if (s_flag[jj])
-                pair_block<SYM, NF, CK, true>(tq, &s_qp[jj * 6], nj.x, nj.y, nj.z, self, k, ki, are, aim, sre, sim);
+                pair_block<SYM, NF, CK, true>(tq, &s_qp[jj * 6], nj.x, nj.y, nj.z, k, ki, are, aim, sre, sim);
             else
-                pair_block<SYM, NF, CK, false>(tq, &s_qp[jj * 6], nj.x, nj.y, nj.z, self, k, ki, are, aim, sre,
-                                               sim);
+                pair_block<SYM, NF, CK, false>(tq, &s_qp[jj * 6], nj.x, nj.y, nj.z, k, ki, are, aim, sre, sim);
             const float scale = HBEM_INV4PI * tjac * nj.w;
             const uchar4 cs = s_cs[jj];
             const int cslot[3] = {cs.x, cs.y, cs.z};
@@ -367,7 +375,7 @@ __global__ void __launch_bounds__(kAsmThreads, MINB) k_regular(const __grid_cons
                     for (int j = 0; j < 3; ++j) {
                         float vre = are[f][i * 3 + j] * scale + radd_re;
                         float vim = aim[f][i * 3 + j] * scale + radd_im;
-                        if (self) vre -= 0.25f * tjac * (i == j ? (1.0f / 6.0f) : (1.0f / 12.0f));
+                        if (self) vre -= 0.25f * tjac * ((i + rot) % 3 == j ? (1.0f / 6.0f) : (1.0f / 12.0f));
                         float2 *dst = &acc[rslot[i] * ldc + cslot[j]];
                         atomicAdd(&dst->x, vre * p.rw);
                         atomicAdd(&dst->y, vim * p.rw);
