@@ -109,6 +109,13 @@ def test_regular_assembly_at_tile_edges(name, freqs, sources, robin):
     _check(name, freqs, sources, robin)
 
 
+@pytest.mark.parametrize("freqs,sources,robin", [(2, 1, False), (3, 3, False), (3, 1, True)])
+@pytest.mark.parametrize("name", sorted(MESHES))
+def test_complex_wavenumbers(name, freqs, sources, robin):
+    """exp(-Im k r) is 2^-22 off, its argument (below 1.5) 2^-23."""
+    _check(name, freqs, sources, robin, damped=True)
+
+
 @pytest.mark.parametrize("freqs,robin,damped", [(1, False, False), (3, True, False), (2, True, True)])
 @pytest.mark.parametrize("name", sorted(set(MESHES) - {"scattered"}))
 def test_ordered_pairs(name, freqs, robin, damped):
