@@ -60,7 +60,8 @@ def test_refined_solution_and_condition_estimate(n, batch):
         assert abs(float(rcond[m]) - want) <= 1e-2 * want
 
 
-HBEM_TUNE_LU_SOLVE = 2
+HBEM_TUNE_LU_SOLVE, HBEM_TUNE_WAVE_SPIN = 2, 7
+HBEM_ERR_STATE = -4
 
 
 @pytest.mark.parametrize("mode", [1, 2, 3])
@@ -94,3 +95,50 @@ def test_forced_solve_schemes_take_the_condition_estimate(mode):
     finally:
         lib.hbem_set_tuning(HBEM_TUNE_LU_SOLVE, 0)
     assert launches[mode] >= launches[0] + 13
+
+
+def test_wait_that_runs_out_is_reported_and_leaves_the_context_usable():
+    """The built-in refinement and condition estimate with their waits bounded to one poll
+    (HBEM_TUNE_WAVE_SPIN = 1): both give up, say so once, and are right again with the built-in bound."""
+    lib = load_library()
+    n = 2048
+    rng = np.random.default_rng(9)
+    A = (rng.standard_normal((1, n, n)) + 1j * rng.standard_normal((1, n, n))).astype(np.complex64)
+    A += (4.0 * np.sqrt(n)) * np.eye(n, dtype=np.complex64)
+    b = (rng.standard_normal((1, n)) + 1j * rng.standard_normal((1, n))).astype(np.complex64)
+    A0r, A0i = _parts(A)
+    Ar, Ai = A0r.clone(), A0i.clone()
+    br, bi = _parts(b)
+    piv = torch.empty((1, n), dtype=torch.int32, device="cuda")
+    info = torch.empty(1, dtype=torch.int32, device="cuda")
+    norm = np.abs(A[0]).sum(0).max().astype(np.float32)
+    anorm = torch.tensor([norm], device="cuda")
+    rcond = torch.empty(1, dtype=torch.float64, device="cuda")
+    st = _stream_ptr()
+    check(lib.hbem_lu_factor(n, 1, _t_ptr(Ar), _t_ptr(Ai), n, n * n, _t_ptr(piv), n, _t_ptr(info), HBEM_PREC_TF32X3,
+                             st), "hbem_lu_factor")
+
+    def estimate():
+        check(lib.hbem_lu_rcond(n, 1, _t_ptr(Ar), _t_ptr(Ai), n, n * n, _t_ptr(anorm), _t_ptr(rcond), st),
+              "hbem_lu_rcond")
+        return lib.hbem_solve_status(st)
+
+    def refine():
+        xr, xi = torch.zeros_like(br), torch.zeros_like(bi)
+        rc = lib.hbem_refine(n, 1, _t_ptr(A0r), _t_ptr(A0i), n, n * n, _t_ptr(Ar), _t_ptr(Ai), n * n, _t_ptr(piv), n,
+                             _t_ptr(br), _t_ptr(bi), n, _t_ptr(xr), _t_ptr(xi), n, 1e-7, 6, None, None, st)
+        return rc, xr.double().cpu().numpy() + 1j * xi.double().cpu().numpy()
+
+    try:
+        check(lib.hbem_set_tuning(HBEM_TUNE_WAVE_SPIN, 1), "hbem_set_tuning")
+        assert estimate() == HBEM_ERR_STATE
+        assert refine()[0] == HBEM_ERR_STATE
+        assert lib.hbem_solve_status(st) == 0   # reported once
+    finally:
+        lib.hbem_set_tuning(HBEM_TUNE_WAVE_SPIN, 0)
+    assert estimate() == 0
+    want, _ = lapack.cgecon(lapack.cgetrf(A[0])[0], norm, norm="1")
+    assert abs(float(rcond[0]) - want) <= 1e-2 * want
+    rc, x = refine()
+    ref = np.linalg.solve(A[0].astype(np.complex128), b[0].astype(np.complex128))
+    assert rc == 0 and np.linalg.norm(x[0] - ref) <= 4e-6 * np.linalg.norm(ref)
