@@ -2853,10 +2853,9 @@ int launch_panel_cluster(float *a_re, float *a_im, long long lda, long long a_st
 
 // CTAs per matrix of the block panel kernel for m rows, 0 when the panel does
 // not fit a cluster.
-int panel_block_ctas(int m, int batch) {
+int panel_block_ctas(int m) {
     const int least = (m + kBlkMaxRows - 1) / kBlkMaxRows;
-    if (least > kBlkMaxCta) return 0;
-    return least;
+    return least > kBlkMaxCta ? 0 : least;
 }
 
 int launch_panel_block(float *a_re, float *a_im, long long lda, long long a_stride, int n, int c, int w, int *piv,
@@ -2968,8 +2967,8 @@ static int lookahead_streams(cudaStream_t key, LookaheadStreams **out) {
 
 // The FP32 LU's look-ahead bulk update on the tensor cores (TF32x3): the
 // built-in choice of HBEM_PREC_TF32X3, or HBEM_TUNE_LU_UPDATE = 2.  Measured
-// on one B200: n = 1043 x 40 factors in 6.5 instead of 7.4 ms, 4096 x 4 in
-// 28.2 instead of 29.6 ms and 18 749 x 2 in 701 instead of 1130 ms; but the
+// on one B200: n = 1044 x 40 factors in 3.7 instead of 5.4 ms, 4096 x 4 in
+// 14.8 instead of 24.5 ms and 18 749 x 2 in 401 instead of 987 ms; but the
 // split products keep 22 of FP32's 24 significand bits, and on a BEM matrix
 // (the 1952-dof quarter horn) the unrefined solution is 5.5e-5 from LAPACK
 // instead of the FP32 LU's < 1e-5.  So HBEM_PREC_PLAIN (cgesv) keeps the
@@ -2982,8 +2981,7 @@ static bool plain_update_on_tensor_cores(int precision) {
 
 int lu_factor(int n, int batch, float *a_re, float *a_im, long long lda, long long a_stride, int *piv,
               long long piv_stride, int *info, int precision, cudaStream_t st) {
-    // Two-level blocking: 64-column blocks (128 for the mixed LU, so its
-    // tensor-core update streams the trailing matrix once per 128 columns)
+    // Two-level blocking: 64-column blocks (128 for the mixed LU on request)
     // whose (n - b0) x NB panel is factored by inner sub-panels (64, 32 or 16
     // wide) with updates confined to the block's columns; then the row swaps,
     // the NB-row TRSM (in 64-row halves) and a K = NB trailing update per block.
@@ -2996,16 +2994,15 @@ int lu_factor(int n, int batch, float *a_re, float *a_im, long long lda, long lo
     // only used on the bulk stream (and on the chain after it has joined).
     const size_t smem_cap = 200 * 1024;
     // 128-column blocks (one K = 128 update per block, half the C stream of
-    // K = 64) pay for large matrices: 18 749 x 2 factors in 417 instead of
-    // 498 ms, 18 749 x 8 in 1460 instead of 1867 ms.  Below that the K = 128
-    // update, whose 128 KB resident A leaves its B ring one 32-column tile
-    // deep, runs at 23 % of HBM where K = 64 reaches 57 % (n = 8192: 2.0 ms
-    // per launch against 0.8 ms for half the K), so 8192 x 4 takes 112 vs
-    // 85 ms and 10 000 x 2 98 vs 83 ms.
+    // K = 64) on request only: their update keeps a 128 KB A, which leaves its
+    // B ring one 32-column tile deep (23 % of HBM at n = 8192 where K = 64
+    // reaches 57 %), and their panels are sub-panels while the 64-column ones
+    // go in whole blocks below 6144 rows.  K = 128 against K = 64: 8192 x 4 86
+    // and 65 ms, 10 000 x 2 91 and 73, 10 000 x 8 255 and 216, 18 749 x 2 409
+    // and 339, 18 749 x 8 1450 and 1267 ms (before whole-block panels K = 128
+    // won the last two, 417 against 498 and 1460 against 1867 ms).
     const int blk_want = tuning(HBEM_TUNE_LU_BLOCK);
-    const int NB = (precision == HBEM_PREC_MIXED && n > 256 && (blk_want == 128 || (blk_want == 0 && n > 16000)))
-                       ? 128
-                       : 64;
+    const int NB = precision == HBEM_PREC_MIXED && n > 256 && blk_want == 128 ? 128 : 64;
     HBEM_CUDA(cudaMemsetAsync(info, 0, sizeof(int) * batch, st));
     // K = 64 block updates on the tensor cores: BF16x3 (mixed precision), or
     // TF32x3 for the plain LU's look-ahead bulk when selected; their barrier
@@ -3117,7 +3114,7 @@ int lu_factor(int n, int batch, float *a_re, float *a_im, long long lda, long lo
     // CTAs of the block panel kernel for a panel of that many rows (0: not this kernel)
     auto block_ctas = [&](int rows) -> int {
         if (!block_panels) return 0;
-        const int ctas = panel_block_ctas(rows, batch);
+        const int ctas = panel_block_ctas(rows);
         return ctas > 0 && panel_block_fits(ctas) ? ctas : 0;
     };
     HBEM_CUDA(cudaFuncSetAttribute(k_swap_trsm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSwapSmem));
@@ -3219,9 +3216,8 @@ int lu_factor(int n, int batch, float *a_re, float *a_im, long long lda, long lo
         const int outside = n - bw;
         const int next_end = std::min(n, b0 + bw + NB);
         // SMs the persistent tensor-core update leaves to the chain (by
-        // default none: with a TF32x3 bulk of two K = 32 passes, leaving 32 SMs
-        // gave n = 1044 x 40 5.98 against 5.87 ms and 1542 x 40 16.4 against
-        // 15.3 ms)
+        // default none: leaving 32 SMs gives n = 1044 x 40 3.96 against 3.73 ms,
+        // 1542 x 40 9.44 against 8.61 and 4096 x 4 14.6 against 14.8 ms)
         const int tc_reserve = tuning(HBEM_TUNE_LU_RESERVE) > 0 ? tuning(HBEM_TUNE_LU_RESERVE) - 1 : 0;
         const bool split = la && next_end < n;
         if (outside > 0) {
