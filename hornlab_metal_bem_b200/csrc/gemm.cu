@@ -774,14 +774,14 @@ template <bool TF32, int KC>
 __global__ void __launch_bounds__(256) k_pack_b(const float *a_re, const float *a_im, long long lda,
                                                 long long a_stride, int start, int col_end, int k0, int cols_pad,
                                                 int cols_used, typename TcSplit<TF32>::T *B2) {
-    // 64 columns per CTA, CH = min(KC, 64) rows of U12 at a time: the CH x 64
+    // 64 columns per CTA, CH = 64 rows of U12 at a time: the CH x 64
     // block is read along its rows (coalesced), transposed in shared memory
     // and written into the packed K-major rows (consecutive threads,
     // consecutive pairs)
     using S = TcSplit<TF32>;
     using T = typename S::T;
     constexpr int K2 = TcCfg<TF32, KC>::K2;
-    constexpr int CH = KC < 64 ? KC : 64, PAIRS = 2 * CH, JSTEP = 256 / PAIRS;
+    constexpr int CH = 64, PAIRS = 2 * CH, JSTEP = 256 / PAIRS;
     __shared__ float s_ur[CH][65], s_ui[CH][65];
     const int mat = blockIdx.z;
     const int j0 = blockIdx.x * 64;
