@@ -40,8 +40,11 @@ import numpy as np
 REPO = Path(__file__).resolve().parent
 sys.path.insert(0, str(REPO))
 
-FLOPS_PER_SAMPLE = 36.0     # algorithmic FP32 flops (FMA = 2) per kernel sample, incl. accumulation
-SFU_PER_SAMPLE = 3.0        # rsqrt, sin, cos
+# per kernel evaluation (point pair, image, wavenumber) of an unordered triangle pair, four images: 12 of the geometry
+# and both dot products (24, shared by two wavenumbers), 7 of e^{ikr} (1/r - ik), 8 for the two orders' values, 9 of the
+# accumulation into both 3 x 3 blocks
+FLOPS_PER_EVAL = 36.0
+SFU_PER_EVAL = 2.5          # sin, cos, and one rsqrt for two wavenumbers
 FP32_LANES_PER_SM = 128
 SFU_LANES_PER_SM = 16
 N_SM = 148
@@ -59,8 +62,7 @@ def parse():
     ap.add_argument("--streams", type=int, default=4, help="c3: concurrent streams")
     ap.add_argument("--precision", choices=["plain", "mixed"], default="plain")
     ap.add_argument("--lu-block", type=int, choices=[0, 32, 64, 128], default=0,
-                    help="lu: column block of the mixed LU, or the K of a TF32x3 bulk pass (HBEM_TUNE_LU_BLOCK; "
-                         "0 = built-in)")
+                    help="lu: column block of the mixed LU (HBEM_TUNE_LU_BLOCK; 0 = built-in 64, 32 acts as 64)")
     ap.add_argument("--lu-update", type=int, choices=[0, 1, 2], default=0,
                     help="lu: plain LU bulk update (HBEM_TUNE_LU_UPDATE; 2 = TF32x3 tensor cores)")
     ap.add_argument("--no-cpu-baseline", action="store_true")
@@ -477,24 +479,22 @@ def run_b200(args, w):
     peaks = measured_peaks()
     m_img = {0: 1, 1: 2, 2: 2, 3: 4, 4: 2}[w["sym"]]
     T = buf.n_triangles
-    samples = F * T * T * 36 * m_img
+    samples = F * T * (T + 1) // 2 * 36 * m_img   # each unordered pair once
     clk_mhz = peaks.get("sm_max_mhz", 1965.0)
     fp32_peak = N_SM * FP32_LANES_PER_SM * 2 * clk_mhz * 1e6 / 1e12
-    achieved = samples * FLOPS_PER_SAMPLE / (stage["regular_ms"] * 1e-3) / 1e12
-    # MUFU pipe: rsqrt, sin, cos once per unordered evaluation, i.e. 1.5 per ordered sample
+    achieved = samples * FLOPS_PER_EVAL / (stage["regular_ms"] * 1e-3) / 1e12
     sfu_peak = N_SM * SFU_LANES_PER_SM * clk_mhz * 1e6
-    sfu_achieved = samples * SFU_PER_SAMPLE / 2 / (stage["regular_ms"] * 1e-3)
+    sfu_achieved = samples * SFU_PER_EVAL / (stage["regular_ms"] * 1e-3)
     roofline = {
         "kernel": "k_regular_sym (regular pair assembly over unordered pairs, %d launch/step)" % ((F + 63) // 64),
         "bound": "fp32", "achieved": achieved, "peak": fp32_peak, "unit": "TFLOP/s", "frac": achieved / fp32_peak,
         "traffic": profile_traffic("k_regular", w["name"]),
-        "algorithmic": f"{samples:.3e} ordered kernel samples/launch x {FLOPS_PER_SAMPLE:.0f} FP32 flops "
-                       "(F T^2 36 M; the kernel evaluates each unordered pair once)",
+        "algorithmic": f"{samples:.3e} kernel evaluations/launch x {FLOPS_PER_EVAL:.0f} FP32 flops "
+                       "(F T (T + 1) / 2 36 M: each unordered pair once, both orders' entries)",
         "peak_source": f"148 SM x 128 FP32 lanes x 2 x {clk_mhz:.0f} MHz (sm_max_mhz, {peaks['source']})",
         "sfu": {"achieved_gops_s": sfu_achieved / 1e9, "peak_gops_s": sfu_peak / 1e9,
                 "frac": sfu_achieved / sfu_peak,
-                "per_sample": "rsqrt + sin + cos (3 MUFU) per unordered evaluation = 1.5 per ordered sample; "
-                              "16 MUFU lanes/clk/SM"},
+                "per_evaluation": "sin + cos, and one rsqrt for two wavenumbers (2.5 MUFU); 16 MUFU lanes/clk/SM"},
     }
     line = {
         "metric": "freq-solves/s", "value": value, "unit": "freq-solves/s", "n_gpus": world, "steps": args.steps,
@@ -614,9 +614,14 @@ def run_b200_c4(args, w, emit: bool = True, accuracy_picks=None, refine_max_iter
     clk_mhz = peaks.get("sm_max_mhz", 1965.0)
     lu_flops = F * (8.0 / 3.0) * N ** 3
     achieved = lu_flops / (stage["solve_ms"] * 1e-3) / 1e12
-    if args.precision == "mixed":
-        peak, pk_src = float(peaks.get("bf16_tflops_sustained", peaks.get("bf16_tflops", 1590.0))), \
-            f"cuBLAS bf16 dense, sustained ({peaks['source']}); BF16x3 issues 3 bf16 products per FP32 product"
+    tensor = args.precision == "mixed" or refine_max_iterations > 0   # refined plain solves: TF32x3 bulk update
+    if tensor:
+        peak = float(peaks.get("bf16_tflops_sustained", peaks.get("bf16_tflops", 1590.0)))
+        pk_src = f"cuBLAS bf16 dense, sustained ({peaks['source']}); BF16x3 issues 3 bf16 products per FP32 product"
+        if args.precision != "mixed":
+            peak *= 0.5
+            pk_src = (f"half of cuBLAS bf16 dense, sustained ({peaks['source']}), the TF32 rate; TF32x3 issues 3 TF32 "
+                      "products per FP32 product")
     else:
         peak = N_SM * FP32_LANES_PER_SM * 2 * clk_mhz * 1e6 / 1e12
         pk_src = f"148 SM x 128 FP32 lanes x 2 x {clk_mhz:.0f} MHz"
@@ -639,7 +644,7 @@ def run_b200_c4(args, w, emit: bool = True, accuracy_picks=None, refine_max_iter
         "accuracy": {"against": "FP64 GPU path: FP64 assembly (A, b, S_ia, S_aa), complex128 LU of the augmented "
                                 "system, FP64 Rayleigh field", "cases": errs},
         "clocks": clk,
-        "roofline": {"kernel": "batched LU + solve of the augmented systems", "bound": "tensor" if args.precision == "mixed" else "fp32",
+        "roofline": {"kernel": "batched LU + solve of the augmented systems", "bound": "tensor" if tensor else "fp32",
                      "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak, "traffic": None,
                      "algorithmic": f"(8/3) N^3 real flops per system, N = {N}, {F} systems", "peak_source": pk_src},
     }

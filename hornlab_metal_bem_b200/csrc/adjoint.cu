@@ -237,8 +237,8 @@ struct BwdArgs {
 // triangle is driven.
 // The trial triangle's gradient is a warp total and the test triangle's stays in
 // registers (per-pair shared atomics, 32 lanes on one address, were a third of
-// the instructions).  Bound: issue, 14 slots of the FP32 pipe per sample and
-// frequency beside the MUFU pipe's sine and cosine.  4160 triangles x 20
+// the instructions).  Bound: issue (73 %; 14 slots of the FMA pipe per sample
+// and frequency, 66 %, beside the MUFU pipe's sine and cosine, 48 %).  4160 triangles x 20
 // frequencies: 40.8 -> 16 ms with the touching pairs.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(kBwdThreads, 2) k_asm_bwd(const __grid_constant__ BwdArgs a) {

@@ -445,9 +445,11 @@ __global__ void __launch_bounds__(kAsmThreads, MINB) k_regular(const __grid_cons
 // one per block entry their retries took half of the kernel with four images
 // and four fifths of it with one.
 //
-// Bound: issue (a packed instruction takes two slots of the FP32 pipe; 82 % of
-// them busy with one image), with four images the MUFU pipe as well (1 rsqrt
-// + 2 NF per sample: 62 %).  Regular assembly with right-hand sides, 40
+// Bound: latency at 12 warps an SM, no pipe at its limit: FMA 64-65 % of its
+// cycles (a packed instruction takes two slots), issue 58-59 %, MUFU (1 rsqrt +
+// 2 NF per sample) 33 % with one image and 62 % with four.  One chunk of many
+// dofs sets the shared memory of the launch: on the full horn below, one chunk
+// of 1042 has 15, which leaves two CTAs an SM (FMA 55 %).  Regular assembly with right-hand sides, 40
 // wavenumbers: quarter horn (1950 triangles, 4 images) 15.8 -> 9.8 ms, half
 // horn (3664, 2 images) 40.0 -> 21.9 ms; full horn (8332, 6 wavenumbers)
 // 26.0 -> 12.2 ms; sphere with every face driven (1280, 8) 2.33 -> 0.74 ms.
@@ -846,8 +848,9 @@ __global__ void __launch_bounds__(kPairWarps * 32, NF == 2 ? 3 : 4) k_regular_sy
 // any of its sources; per triangle the six points and their images give one
 // complex sum per wavenumber (NF share the geometry), which every source
 // multiplies by its q.  The points' totals are contracted with the basis and
-// added to b per test row at the end.  Sums are nested (triangle, 32
-// triangles, CTA) so that each adds few terms.  Done apart from the matrix:
+// added to b per test row at the end.  Bound where every face is driven: MUFU
+// (85 % of its cycles, 1280 triangles x 8 wavenumbers).  Sums are nested
+// (triangle, 32 triangles, CTA) so that each adds few terms.  Done apart from the matrix:
 // only driven triangles need G, and no 3 x 3 blocks are formed for it.
 // ---------------------------------------------------------------------------
 constexpr int kRhsTrials = 256;   // at most; fewer (p.rhs_block) when that leaves SMs idle

@@ -195,8 +195,10 @@ int launch_trailing_update(int n, int batch, int k0, int kw, int start, int col_
 //           and wrote C twice per 64-column block; the whole factorisation
 //           took (two K = 32 passes -> this) 1043 x 40 4.75 -> 3.72 ms, 1900 x
 //           20 10.2 -> 7.6, 4217 x 2 14.6 -> 12.0, 4217 x 6 27.6 -> 19.7, 8000 x
-//           2 59 -> 45, 14 000 x 1 152 -> 115 ms.  Bound by the tensor pipe's
-//           TF32 rate and C's read-modify-write together.
+//           2 59 -> 45, 14 000 x 1 152 -> 115 ms.  On 1044 x 40 and 4217 x 2 the
+//           tensor pipe is 33-34 % active and C's read-modify-write moves 3.0-3.4
+//           TB/s, half of a copy's rate: neither is at its limit, what is left
+//           is the latency of a tile's chain (C in, products, C out).
 // Every mbarrier wait is bounded; a timeout sets the status word and the CTA
 // returns after releasing its TMEM.
 // ===========================================================================
