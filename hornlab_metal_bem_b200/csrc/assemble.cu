@@ -519,7 +519,10 @@ __device__ __forceinline__ void pair_accumulate(const float4 *__restrict__ tq, c
                 const int mk = image_mask<SYM>(m);
                 const float dx = sgn(mk, 0) * y.x - x.x, dy = sgn(mk, 1) * y.y - x.y, dz = sgn(mk, 2) * y.z - x.z;
                 // 1e-30 leaves r^2 of distinct points unchanged in FP32 and
-                // keeps the coincident point finite (its factors are 0)
+                // keeps the coincident point finite (its factors are 0).  The
+                // other kernels' r^2 > 1e-14 would cost 2-3 % of a sweep here
+                // (1043 x 40 22.8 -> 23.3 ms, 1900 x 40 53.3 -> 54.8); it
+                // differs for points less than 1e-7 m apart but not coincident
                 const float r2 = fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, 1.0e-30f)));
                 const float u = rsqrt_ftz(r2);
                 const float r = r2 * u, us = u * u * scale;
