@@ -8,7 +8,7 @@
 //     k_panel_block  : the whole block in one CTA or cluster, rows in place;
 //     k_move_solve   : its net row moves and U12 = L11^-1 A12;
 //     trailing       : A22 -= L21 U12 with K = 64.
-// HBEM_PREC_PLAIN, taller blocks and the HBEM_TUNE_LU_PANEL widths:
+// HBEM_PREC_PLAIN, taller blocks and the HBEM_TUNE_LU_PANEL / _PANEL_KERNEL choices:
 //   for each 64-column block b0:
 //     for each inner sub-panel c (64, 32 or 16 columns):
 //       k_panel      : factor rows c..n of the sub-panel with partial pivoting
