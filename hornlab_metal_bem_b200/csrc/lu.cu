@@ -2981,7 +2981,8 @@ static bool plain_update_on_tensor_cores(int precision) {
 
 int lu_factor(int n, int batch, float *a_re, float *a_im, long long lda, long long a_stride, int *piv,
               long long piv_stride, int *info, int precision, cudaStream_t st) {
-    // Two-level blocking: 64-column blocks (128 for the mixed LU on request)
+    // Two-level blocking: 64-column blocks (128 for the mixed LU, so its
+    // tensor-core update streams the trailing matrix once per 128 columns)
     // whose (n - b0) x NB panel is factored by inner sub-panels (64, 32 or 16
     // wide) with updates confined to the block's columns; then the row swaps,
     // the NB-row TRSM (in 64-row halves) and a K = NB trailing update per block.
@@ -2994,15 +2995,17 @@ int lu_factor(int n, int batch, float *a_re, float *a_im, long long lda, long lo
     // only used on the bulk stream (and on the chain after it has joined).
     const size_t smem_cap = 200 * 1024;
     // 128-column blocks (one K = 128 update per block, half the C stream of
-    // K = 64) on request only: their update keeps a 128 KB A, which leaves its
-    // B ring one 32-column tile deep (23 % of HBM at n = 8192 where K = 64
-    // reaches 57 %), and their panels are sub-panels while the 64-column ones
-    // go in whole blocks below 6144 rows.  K = 128 against K = 64: 8192 x 4 86
-    // and 65 ms, 10 000 x 2 91 and 73, 10 000 x 8 255 and 216, 18 749 x 2 409
-    // and 339, 18 749 x 8 1450 and 1267 ms (before whole-block panels K = 128
-    // won the last two, 417 against 498 and 1460 against 1867 ms).
+    // K = 64) for large matrices: with rows of an odd pitch 18 749 x 2 takes
+    // 415 instead of 488 ms, 18 749 x 8 1460 instead of 1867.  Rows on 16 bytes
+    // (the sweep paths) turn it round at every size: 18 749 x 2 409 ms against
+    // 335 with K = 64, 18 749 x 8 1450 against 1267, 10 000 x 8 255 against 216,
+    // 10 000 x 2 91 against 73, 8192 x 4 86 against 65 (the K = 128 update keeps
+    // a 128 KB A, which leaves its B ring one 32-column tile deep: 23 % of HBM
+    // at n = 8192 where K = 64 reaches 57 %); the rule does not look at the pitch.
     const int blk_want = tuning(HBEM_TUNE_LU_BLOCK);
-    const int NB = precision == HBEM_PREC_MIXED && n > 256 && blk_want == 128 ? 128 : 64;
+    const int NB = (precision == HBEM_PREC_MIXED && n > 256 && (blk_want == 128 || (blk_want == 0 && n > 16000)))
+                       ? 128
+                       : 64;
     HBEM_CUDA(cudaMemsetAsync(info, 0, sizeof(int) * batch, st));
     // K = 64 block updates on the tensor cores: BF16x3 (mixed precision), or
     // TF32x3 for the plain LU's look-ahead bulk when selected; their barrier
@@ -3092,9 +3095,9 @@ int lu_factor(int n, int batch, float *a_re, float *a_im, long long lda, long lo
     // sub-panels held in registers, one row per thread (64 columns up to 384
     // rows, 32 up to 768, 16 up to 1024), when asked for; false: use the
     // shared-memory or cluster kernels.  Not the default: on one B200 the
-    // n = 1043 x 40 factorisation takes 6.69 ms with them against 6.56 ms
-    // (TF32x3 bulk; 7.50 against 7.47 ms with the CUDA-core bulk).  Either
-    // kind costs about 2.4 us per column, which is the two CTA barriers and
+    // n = 1043 x 40 factorisation took 6.69 ms with them against 6.56 ms with
+    // shared-memory sub-panels (TF32x3 bulk; 7.50 against 7.47 ms with the
+    // CUDA-core bulk; whole-block panels 3.73).  Either kind of sub-panel costs about 2.4 us per column, which is the two CTA barriers and
     // the pivot-row exchange of every column, not the row traffic that the
     // registers remove.
     auto panel_in_registers = [&](int c, int w) -> bool {

@@ -140,8 +140,9 @@ long long hbem_launch_count(void);
  *                            split products, for both)
  *   HBEM_TUNE_LU_BLOCK:      column block of the mixed (BF16x3) LU and the K
  *                            of its tensor-core update (64 or 128; 0: the
- *                            built-in 64; 32 is accepted and acts as 64); the
- *                            FP32 LU's TF32x3 bulk takes K = 64 with any value
+ *                            built-in 128 for n > 16000, else 64; 32 is
+ *                            accepted and acts as 64); the FP32 LU's TF32x3
+ *                            bulk takes K = 64 with any value
  *   HBEM_TUNE_LU_PANEL_KERNEL: sub-panels with their rows in shared memory
  *                            (0, built-in) or, where one row per thread fits,
  *                            in registers (1: 64 columns up to 384 rows, 32
