@@ -58,8 +58,8 @@ def test_either_tile_gives_the_same_bits(name):
 
 
 def test_fewer_points_take_no_longer():
-    """Quarter horn, one frequency: just below two CTAs of eight points an SM against just there.  Medians of 15
-    timings of 8 calls each, in turn; they repeat within 1 %."""
+    """Quarter horn, one frequency: just below two CTAs of eight points an SM against just there.  The fastest of
+    15 timings of 8 calls each, in turn; they repeat within 1 %."""
     with _session("quarter") as s:
         data = _data(s)
         sm = torch.cuda.get_device_properties(0).multi_processor_count
@@ -76,5 +76,5 @@ def test_fewer_points_take_no_longer():
                 torch.cuda.synchronize()
                 if rep >= 2:
                     times[i].append(e0.elapsed_time(e1))
-        fewer, more = (float(np.median(t)) for t in times)
+        fewer, more = (min(t) for t in times)
         assert fewer <= 1.03 * more
